@@ -92,7 +92,7 @@ struct ProgMirror {
 };
 
 struct prism_handle {
-  DevBuf qc, planes, status, offs, bsum, part, wins, ranges, anchors, small, dev_in, dev_out, zero_anchors;
+  DevBuf qc, planes, status, offs, part, wins, ranges, anchors, small, dev_in, dev_out, zero_anchors;
   DevBuf qc_odd;  // the code buffer of a progressive object's odd-numbered steps
   DevBuf ext;     // per-CTA partials of the extrema scan
   DevBuf sbatch;  // batched strategy searches: cells, inputs and states
@@ -135,7 +135,7 @@ struct prism_handle {
   uint64_t prog_used = 0;
   ProgMirror* prog_host = nullptr;  // 64 mapped mirrors, one per slot
   ProgMirror* prog_host_dev = nullptr;
-  // per slot: the chunk offsets of the slot's container, computed by its
+  // per slot: the chunk table of the slot's container, computed by its
   // first step and reused by the later ones
   DevBuf prog_offs[64];
   size_t zero_anchors_ready = 0;  // leading bytes of zero_anchors known to be zero
@@ -235,7 +235,7 @@ struct prism_prog {
   StrategyState* d_state = nullptr;
   int* d_err = nullptr;         // chunk errors of every step so far
   int slot = -1;                // slot in the handle's state block, or -1 (own allocation)
-  bool offs_ready = false;      // the slot's chunk offsets hold this container's
+  bool offs_ready = false;      // the slot's chunk table holds this container's
   ProgMirror* mirror = nullptr;      // mapped host copy written by each step
   ProgMirror* mirror_dev = nullptr;
   uint64_t loaded = 0;          // host copy, valid when !pending
@@ -341,8 +341,7 @@ static int ensure_common(prism_handle* h, const Geometry& g) {
   CKA(h->qc.ensure(qc_len(g) * sizeof(int32_t)));
   CKA(h->planes.ensure(g.aligned_size + 64));
   CKA(h->status.ensure((size_t)g.chunks * sizeof(unsigned long long)));
-  CKA(h->offs.ensure((size_t)g.chunks * sizeof(int64_t) + 64));
-  CKA(h->bsum.ensure(((size_t)g.chunks / kScanItems + 2) * sizeof(int64_t)));
+  CKA(h->offs.ensure(chunk_table_bytes(g.chunks)));
   CKA(h->anchors.ensure(g.anchors * 8 + 64));
   CKA(h->small.ensure(sizeof(Small)));
   return PRISM_OK;
@@ -479,8 +478,10 @@ static int launch_bitshuffle(prism_handle* h, const int32_t* qc, const Geometry&
   return PRISM_OK;
 }
 
+// live: the dead chunks of `planes` (written by launch_decode with the same
+// one), which are not read
 static int launch_inverse(prism_handle* h, const uint8_t* planes, const Geometry& g, int nb, const int* dbegin,
-                          const int* dend, int32_t* qc, cudaStream_t st) {
+                          const int* dend, const ChunkLive& live, int32_t* qc, cudaStream_t st) {
   int64_t start_last = (g.sh_grid - 1) * (int64_t)kChunk;
   // positions from the last block on are only partly written: start from 0
   uint64_t from = g.anchors + (uint64_t)start_last;
@@ -491,10 +492,12 @@ static int launch_inverse(prism_handle* h, const uint8_t* planes, const Geometry
   prof_begin(h, kStInverse, st);
   if (plan.items > 0) {
     int64_t blocks = (plan.items + kShufWarps - 1) / kShufWarps;
-    inverse_bitshuffle_kernel<<<(unsigned)blocks, kShufWarps * 32, 0, st>>>(planes, codes, g, plan, nb, dbegin, dend);
+    inverse_bitshuffle_kernel<<<(unsigned)blocks, kShufWarps * 32, 0, st>>>(planes, codes, g, plan, nb, dbegin, dend,
+                                                                             live);
     h->launches += 1;
   }
-  inverse_last_block_kernel<<<last_block_rounds(g), 512, 0, st>>>(planes, codes, g, nb, dbegin, dend, g.aligned_size);
+  inverse_last_block_kernel<<<last_block_rounds(g), 512, 0, st>>>(planes, codes, g, nb, dbegin, dend, g.aligned_size,
+                                                                    live);
   prof_end(h, kStInverse, st);
   h->launches += 1;
   CK(cudaGetLastError());
@@ -526,37 +529,48 @@ static int launch_encode(prism_handle* h, const uint8_t* planes, const Geometry&
   return PRISM_OK;
 }
 
-// err: where chunk errors go; null = the handle's flag, reset here
-// payload offset of every chunk: exclusive prefix sum of the size table
-static void launch_chunk_offsets(prism_handle* h, const uint8_t* stream, const Geometry& g, int64_t* offs,
-                                 cudaStream_t st) {
-  const uint16_t* sizes = reinterpret_cast<const uint16_t*>(stream + 8);
-  int64_t nblk = (g.chunks + kScanItems - 1) / kScanItems;
-  scan_sizes_block<<<(unsigned)nblk, 1024, 0, st>>>(sizes, g.chunks, offs, h->bsum.as<int64_t>());
-  scan_block_sums<<<1, 32, 0, st>>>(h->bsum.as<int64_t>(), nblk);
-  scan_add<<<(unsigned)((g.chunks + 255) / 256), 256, 0, st>>>(offs, g.chunks, h->bsum.as<int64_t>());
-  h->launches += 3;
+// payload offsets and coded chunks of a stream (ChunkTable in `table`)
+static void launch_chunk_table(prism_handle* h, const uint8_t* stream, const Geometry& g, void* table,
+                               cudaStream_t st) {
+  const int64_t blocks = (g.chunks + kScanItems - 1) / kScanItems;
+  scan_chunks_kernel<<<(unsigned)blocks, kScanThreads, 0, st>>>(reinterpret_cast<const uint16_t*>(stream + 8), g,
+                                                                chunk_table(table, g.chunks));
+  h->launches += 1;
 }
 
-// offs_in: chunk offsets already computed for this stream (else computed here)
+// The chunks of a stream an inverse shuffle need not read after launch_decode
+// of the planes [dbegin, dend) (null: all).
+static ChunkLive chunk_live(const uint8_t* stream, const int* dbegin, const int* dend) {
+  return ChunkLive{reinterpret_cast<const uint16_t*>(stream + 8), dbegin, dend};
+}
+
+// edges: the planes are only read through chunk_live, so dead chunks are left
+// alone but for their edges.  err: where chunk errors go; null = the handle's
+// flag, reset here.  table: the stream's chunk table if already built (else
+// built here).
 static int launch_decode(prism_handle* h, const uint8_t* stream, uint64_t stream_bytes, const Geometry& g,
-                         const int* dbegin, const int* dend, uint8_t* planes, cudaStream_t st, int* err = nullptr,
-                         const int64_t* offs_in = nullptr) {
+                         const int* dbegin, const int* dend, uint8_t* planes, bool edges, cudaStream_t st,
+                         int* err = nullptr, void* table = nullptr) {
   Small* s = small(h);
   prof_begin(h, kStDecode, st);
-  const int64_t* offs = offs_in;
-  if (!offs) {
-    launch_chunk_offsets(h, stream, g, h->offs.as<int64_t>(), st);
-    offs = h->offs.as<int64_t>();
+  if (!table) {
+    table = h->offs.p;
+    launch_chunk_table(h, stream, g, table, st);
   }
   if (!err) {
     err = &s->error_flag;
     CK(cudaMemsetAsync(err, 0, sizeof(int), st));
   }
   size_t smem = sizeof(DecodeShared);
-  CK(smem_limit<zbpc_decode_kernel>((int)smem));
-  int blocks = (int)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * 8);
-  zbpc_decode_kernel<<<blocks, kZThreads, smem, st>>>(stream, stream_bytes, offs, g, planes, dbegin, dend, err);
+  int blocks = (int)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * kDecCtas);
+  const ChunkTable t = chunk_table(table, g.chunks);
+  if (edges) {
+    CK(smem_limit<zbpc_decode_kernel<true>>((int)smem));
+    zbpc_decode_kernel<true><<<blocks, kDecThreads, smem, st>>>(stream, stream_bytes, t, g, planes, dbegin, dend, err);
+  } else {
+    CK(smem_limit<zbpc_decode_kernel<false>>((int)smem));
+    zbpc_decode_kernel<false><<<blocks, kDecThreads, smem, st>>>(stream, stream_bytes, t, g, planes, dbegin, dend, err);
+  }
   prof_end(h, kStDecode, st);
   h->launches += 1;
   CK(cudaGetLastError());
@@ -665,9 +679,10 @@ static int decompress_t(prism_handle* h, const uint8_t* cont, uint64_t size, con
   CK(cudaMemcpyAsync(&s->range, tr + 8, sizeof(double), cudaMemcpyDeviceToDevice, st));
   params_kernel<T><<<1, 32, 0, st>>>(mode, bound, &s->range, alpha_of(mode == 1 ? bound : 0.0), nullptr, 0, tr, 4,
                                      reinterpret_cast<PredParams<T>*>(s->params), nullptr, &s->eb);
-  rc = launch_decode(h, cont, size - g.header_size, g, nullptr, nullptr, h->planes.as<uint8_t>(), st);
+  rc = launch_decode(h, cont, size - g.header_size, g, nullptr, nullptr, h->planes.as<uint8_t>(), true, st);
   if (rc) return rc;
-  rc = launch_inverse(h, h->planes.as<uint8_t>(), g, 0 /*SM*/, nullptr, nullptr, h->qc.as<int32_t>(), st);
+  rc = launch_inverse(h, h->planes.as<uint8_t>(), g, 0 /*SM*/, nullptr, nullptr, chunk_live(cont, nullptr, nullptr),
+                      h->qc.as<int32_t>(), st);
   if (rc) return rc;
   prof_begin(h, kStReconstruct, st);
   rc = launch_reconstruct<T, false>(h, h->qc.as<int32_t>(), reinterpret_cast<const T*>(tr + 1040), g,
@@ -699,7 +714,7 @@ int prism_create(prism_handle** out) {
 
 void prism_destroy(prism_handle* h) {
   if (!h) return;
-  DevBuf* bufs[] = {&h->qc, &h->planes, &h->status, &h->offs, &h->bsum, &h->part, &h->wins, &h->ranges,
+  DevBuf* bufs[] = {&h->qc, &h->planes, &h->status, &h->offs, &h->part, &h->wins, &h->ranges,
                     &h->anchors, &h->small, &h->dev_in, &h->dev_out, &h->zero_anchors, &h->prog_slots,
                     &h->sbatch, &h->qc_odd, &h->ext};
   for (DevBuf* b : bufs) b->release();
@@ -1010,26 +1025,28 @@ static int progressive_step_t(prism_prog* p, double target, const T* prev, T* va
                                          p->exact ? s->dec_begin : nullptr);
   prof_end(h, kStStrategy, dst);
   h->launches += 2;
-  // chunk offsets: once per object when it holds a slot
-  const int64_t* offs = nullptr;
+  // chunk table: once per object when it holds a slot
+  void* table = nullptr;
   if (p->slot >= 0) {
     DevBuf& ob = h->prog_offs[p->slot];
     if (!p->offs_ready) {
-      CKA(ob.ensure(((size_t)g.chunks + 1) * sizeof(int64_t)));
-      launch_chunk_offsets(h, p->cont, g, ob.as<int64_t>(), dst);
+      CKA(ob.ensure(chunk_table_bytes(g.chunks)));
+      launch_chunk_table(h, p->cont, g, ob.p, dst);
       p->offs_ready = true;
     }
-    offs = ob.as<int64_t>();
+    table = ob.p;
   }
-  // chunks of planes the step does not load are written as zeros; the
-  // inverse shuffle keeps planes [begin, end) of what was decoded
-  rc = launch_decode(h, p->cont, p->size - g.header_size, g, p->exact ? s->dec_begin : ds->begin, ds->end,
-                     h->planes.as<uint8_t>(), dst, p->d_err, offs);
+  // chunks of planes the step does not load read as zeros; the inverse
+  // shuffle keeps planes [begin, end) of what was decoded
+  const int* dec_begin = p->exact ? s->dec_begin : ds->begin;
+  rc = launch_decode(h, p->cont, p->size - g.header_size, g, dec_begin, ds->end, h->planes.as<uint8_t>(), true, dst,
+                     p->d_err, table);
   if (rc) return rc;
   // the state after the step (plane ranges, errors, bytes loaded) for the host
   prog_publish_kernel<<<1, 32, 0, dst>>>(ds, p->d_err, csbp, p->mirror_dev);
   h->launches += 1;
-  rc = launch_inverse(h, h->planes.as<uint8_t>(), g, 1 /*NB*/, ds->begin, ds->end, codes, dst);
+  rc = launch_inverse(h, h->planes.as<uint8_t>(), g, 1 /*NB*/, ds->begin, ds->end,
+                      chunk_live(p->cont, dec_begin, ds->end), codes, dst);
   if (rc) return rc;
   CK(cudaEventRecord(h->dec_done, dst));
   // ---- on the caller's stream: reconstruction
@@ -1288,7 +1305,7 @@ int prism_inverse_bitshuffle(prism_handle* h, const uint8_t* d_planes, uint32_t 
   int *db, *de;
   rc = host_range(h, begin, end, st, &db, &de);
   if (rc) return rc;
-  rc = launch_inverse(h, d_planes, g, progressive ? 1 : 0, db, de, d_codes, st);
+  rc = launch_inverse(h, d_planes, g, progressive ? 1 : 0, db, de, ChunkLive{}, d_codes, st);
   if (rc) return rc;
   CK(cudaStreamSynchronize(st));
   return PRISM_OK;
@@ -1394,7 +1411,7 @@ int prism_lossless_decode(prism_handle* h, const uint8_t* d_stream, uint32_t nx,
   int *db, *de;
   rc = host_range(h, begin, end, st, &db, &de);
   if (rc) return rc;
-  rc = launch_decode(h, d_stream, ~0ull, g, db, de, d_planes, st);
+  rc = launch_decode(h, d_stream, ~0ull, g, db, de, d_planes, false, st);
   if (rc) return rc;
   return finish(h, st);
 }

@@ -367,100 +367,231 @@ __global__ void zbpc_finish_kernel(uint8_t* stream, Geometry g, const uint64_t* 
 }
 
 // ---------------- decode ----------------
-// exclusive scan of the uint16 size table into int64 offsets (3 kernels)
-constexpr int kScanItems = 4096;
+// Per-chunk tables of a stream, derived from its size table:
+//   coded[k] the k-th coded chunk; an all-zero chunk is 2 bytes, every other
+//            chunk has another size (a chunk spans at least 8 bytes)
+//   offs[i]  payload offset of chunk i (exclusive prefix sum of the sizes)
+//   rank[i]  coded chunks before chunk i (rank[n] = all of them), so the coded
+//            chunks of an id range [s, e) are coded[rank[s] .. rank[e])
+// A coded entry holds the payload offset and size and the plane-buffer offset
+// and size of its chunk (48 + 16 bits each): one 16-byte load tells a CTA
+// all it needs.
+struct ChunkTable {
+  ulonglong2* coded;
+  int64_t* offs;
+  uint32_t* rank;
+};
+__host__ __device__ __forceinline__ ChunkTable chunk_table(void* p, int64_t n) {
+  ChunkTable t;
+  t.coded = reinterpret_cast<ulonglong2*>(p);
+  t.offs = reinterpret_cast<int64_t*>(t.coded + n);
+  t.rank = reinterpret_cast<uint32_t*>(t.offs + n);
+  return t;
+}
+constexpr int kChunkTableBytes = 28;  // per chunk
+inline size_t chunk_table_bytes(int64_t n) { return (size_t)n * kChunkTableBytes + 64; }
+__device__ __forceinline__ ulonglong2 pack_coded(uint64_t off, uint32_t csize, uint64_t base, uint32_t osize) {
+  return make_ulonglong2(off | (uint64_t)csize << 48, base | (uint64_t)osize << 48);
+}
+constexpr uint64_t kCodedMask = (1ull << 48) - 1;
 
-__global__ void __launch_bounds__(1024) scan_sizes_block(const uint16_t* __restrict__ sizes, int64_t n,
-                                                         int64_t* __restrict__ offs, int64_t* __restrict__ block_sum) {
-  __shared__ int64_t warp_tot[32];
-  int64_t base = (int64_t)blockIdx.x * kScanItems + threadIdx.x * 4;
-  int64_t v[4];
-  int64_t s = 0;
+constexpr uint32_t kZeroChunkBytes = 2;
+constexpr int kScanThreads = 1024, kScanPer = 4, kScanItems = kScanThreads * kScanPer;
+
+// One launch for the whole table: a CTA scans kScanItems sizes and gets the
+// sums before them by reading the earlier part of the table itself (16 bits a
+// chunk: 0.5 MB for a 4.3 GB field, from L2), which costs less than a second
+// launch or a wait on the CTAs before it.
+__global__ void __launch_bounds__(kScanThreads)
+scan_chunks_kernel(const uint16_t* __restrict__ sizes, Geometry g, ChunkTable t) {
+  __shared__ unsigned long long warp_tot[32], prior_b[32];
+  __shared__ unsigned prior_c[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t n = g.chunks, base = (int64_t)blockIdx.x * kScanItems;
+  const bool vec = (reinterpret_cast<uintptr_t>(sizes) & 7) == 0;  // four sizes a load
+  auto four = [&](int64_t i, uint32_t (&v)[4]) {
+    if (vec && i + 4 <= n) {
+      const uint2 q = __ldg(reinterpret_cast<const uint2*>(sizes + i));
+      v[0] = q.x & 0xffffu;
+      v[1] = q.x >> 16;
+      v[2] = q.y & 0xffffu;
+      v[3] = q.y >> 16;
+    } else {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) { v[k] = base + k < n ? sizes[base + k] : 0; s += v[k]; }
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int64_t incl = s;
+      for (int k = 0; k < 4; ++k) v[k] = i + k < n ? sizes[i + k] : kZeroChunkBytes;
+    }
+  };
+  const int64_t i0 = base + (int64_t)tid * kScanPer;
+  uint32_t v[kScanPer];
+  four(i0, v);
+  unsigned long long pb = 0;
+  unsigned pc = 0;
+#pragma unroll 8
+  for (int64_t i = 4 * tid; i < base; i += 4 * kScanThreads) {
+    uint32_t w[4];
+    four(i, w);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      pb += w[k];
+      pc += w[k] != kZeroChunkBytes;
+    }
+  }
+  unsigned long long own = 0;  // bytes (below 2^32 for a CTA's chunks), coded chunks << 32
+#pragma unroll
+  for (int k = 0; k < kScanPer; ++k) own += v[k] | (unsigned long long)(v[k] != kZeroChunkBytes) << 32;
+  unsigned long long incl = own;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    int64_t t = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += t;
+    const unsigned long long x = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += x;
   }
-  if (lane == 31) warp_tot[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    int64_t w = warp_tot[lane];
-    int64_t wi = w;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      int64_t t = __shfl_up_sync(0xffffffffu, wi, d);
-      if (lane >= d) wi += t;
+  for (int d = 16; d > 0; d >>= 1) pb += __shfl_xor_sync(0xffffffffu, pb, d);
+  pc = __reduce_add_sync(0xffffffffu, pc);
+  if (lane == 31) {
+    warp_tot[warp] = incl;
+    prior_b[warp] = pb;
+    prior_c[warp] = pc;
+  }
+  __syncthreads();
+  unsigned long long before = lane < warp ? warp_tot[lane] : 0;
+  pb = prior_b[lane];
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    before += __shfl_xor_sync(0xffffffffu, before, d);
+    pb += __shfl_xor_sync(0xffffffffu, pb, d);
+  }
+  pc = __reduce_add_sync(0xffffffffu, prior_c[lane]);
+  before += incl - own;
+  unsigned long long off = pb + (before & 0xffffffffu);
+  uint32_t rank = pc + (uint32_t)(before >> 32);
+#pragma unroll
+  for (int k = 0; k < kScanPer; ++k) {
+    const int64_t i = i0 + k;
+    if (i < n) {
+      t.offs[i] = (int64_t)off;
+      t.rank[i] = rank;
+      if (v[k] != kZeroChunkBytes) {
+        const ChunkLoc loc = locate_chunk(g, i);
+        t.coded[rank++] = pack_coded(off, v[k], (uint64_t)loc.base, (uint32_t)loc.osize);
+      }
+      off += v[k];
+      if (i == n - 1) t.rank[n] = rank;
     }
-    warp_tot[lane] = wi - w;
-    if (lane == 31) block_sum[blockIdx.x] = wi;
-  }
-  __syncthreads();
-  int64_t run = warp_tot[warp] + incl - s;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (base + k < n) offs[base + k] = run;
-    run += v[k];
   }
 }
 
-__global__ void scan_block_sums(int64_t* block_sum, int64_t nblocks) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    int64_t acc = 0;
-    for (int64_t i = 0; i < nblocks; ++i) { int64_t t = block_sum[i]; block_sum[i] = acc; acc += t; }
-  }
-}
-
-__global__ void scan_add(int64_t* offs, int64_t n, const int64_t* block_sum) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) offs[i] += block_sum[i / kScanItems];
-}
+constexpr int kDecThreads = 256, kDecWarps = kDecThreads / 32;
+constexpr int kDecCtas = 6;  // per SM
 
 struct DecodeShared {
   uint8_t in[kChunk + 32];
-  uint8_t bm0[2048];
+  uint4 out[kDecWarps][64];  // 1024 decoded bytes of each warp, on their way to coalesced stores
+  uint32_t expand[16];
   uint8_t bm1[256];
-  uint8_t bm2[32];
-  int scratch[40];
-  int flag;
+  int scan1[kDecWarps], scan2[kDecWarps];
+  int p2, flag;
 };
 
-// Copy n <= kChunk bytes from an arbitrarily aligned global address into
-// shared memory with aligned 32-bit loads; no byte past src + n - 1's word is
-// read.  A thread's words are w = t + k * kZThreads (k < 8); every load is
-// issued before the first store, so a chunk costs one load latency.  Each
-// source word is loaded once: the word after w is the next lane's (lane 31
-// loads it itself).
-__device__ __forceinline__ void copy_in(uint8_t* dst, const uint8_t* src, int n) {
-  constexpr int kWords = kChunk / 4 / kZThreads;
+// Copy n <= kChunk bytes from an arbitrarily aligned global address to `dst`
+// (shared memory, or global memory for a raw chunk) with aligned 32-bit
+// loads; no byte past src + n - 1's word is read.  Four words a thread are in
+// flight.  Each source word is loaded once: the word after w is the next
+// lane's (lane 31 loads it itself).  Whole words are written (n is a multiple
+// of 4 for raw chunks; the staging buffer has slack).
+__device__ __forceinline__ void copy_words(uint32_t* dw, const uint8_t* src, int n) {
   const int shift = (int)((uintptr_t)src & 3);
   const uint32_t* a = reinterpret_cast<const uint32_t*>(src - shift);
   const int last = (shift + n - 1) >> 2;  // last source word needed
   const int lane = threadIdx.x & 31;
-  uint32_t* dw = reinterpret_cast<uint32_t*>(dst);
-  uint32_t lo[kWords], hi[kWords];
+#pragma unroll 1
+  for (int w0 = threadIdx.x; 4 * (w0 - lane) < n; w0 += 4 * kDecThreads) {  // warp-uniform trips
+    uint32_t lo[4], hi[4];
 #pragma unroll
-  for (int k = 0; k < kWords; ++k) {
-    const int w = threadIdx.x + k * kZThreads;
-    lo[k] = w <= last ? __ldg(a + w) : 0u;
-    hi[k] = (lane == 31 && w + 1 <= last) ? __ldg(a + w + 1) : 0u;
-  }
+    for (int k = 0; k < 4; ++k) {
+      const int w = w0 + k * kDecThreads;
+      lo[k] = w <= last ? __ldg(a + w) : 0u;
+      hi[k] = (lane == 31 && w + 1 <= last) ? __ldg(a + w + 1) : 0u;
+    }
 #pragma unroll
-  for (int k = 0; k < kWords; ++k) {
-    const int w = threadIdx.x + k * kZThreads;
-    const uint32_t next = __shfl_down_sync(0xffffffffu, lo[k], 1);
-    if (lane != 31) hi[k] = next;
-    if (4 * w < n) dw[w] = shift ? __funnelshift_r(lo[k], hi[k], 8 * shift) : lo[k];
+    for (int k = 0; k < 4; ++k) {
+      const int w = w0 + k * kDecThreads;
+      const uint32_t next = __shfl_down_sync(0xffffffffu, lo[k], 1);
+      if (lane != 31) hi[k] = next;
+      if (4 * w < n) dw[w] = __funnelshift_r(lo[k], hi[k], 8 * shift);
+    }
   }
+}
+
+// Exclusive prefix of two counts below 2^16 packed in `v`, one word of 32
+// bitmap bits each: the thread's word of the warp's first 32 words (low half)
+// and of its second 32 (high half); a warp's 64 words follow the previous
+// warp's.  One barrier; `scratch` must not be in use since the last one.
+struct TwoRanks {
+  int first, second, total;
+};
+__device__ __forceinline__ TwoRanks block_two_ranks(uint32_t v, int* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+  const int tf = (int)(all & 0xffffu), ts = (int)(all >> 16);
+  if (lane == 0) scratch[warp] = tf + ts;
+  __syncthreads();
+  const int t = lane < kDecWarps ? scratch[lane] : 0;
+  const int before = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < warp ? t : 0));
+  TwoRanks r;
+  r.total = (int)__reduce_add_sync(0xffffffffu, (unsigned)t);
+  const uint32_t excl = incl - v;
+  r.first = before + (int)(excl & 0xffffu);
+  r.second = before + tf + (int)(excl >> 16);
+  return r;
+}
+
+// The 32 plane bytes whose nonzero flags are `bits`, the kept ones from
+// in[rank] on, into this lane's part of the warp's staging (16-byte pieces
+// swizzled so that eight lanes touch eight bank groups).  Few bytes are
+// stored one by one; otherwise four bytes at a time, the next kept bytes
+// placed by one byte permute whose selector comes from a 16-entry table.
+__device__ __forceinline__ int stage_piece(int p) { return p ^ ((p >> 3) & 1); }
+__device__ __forceinline__ void expand_word(const DecodeShared& sh, uint4* stage, uint32_t bits, int rank, int most) {
+  const int lane = threadIdx.x & 31;
+  uint4 &p0 = stage[stage_piece(2 * lane)], &p1 = stage[stage_piece(2 * lane + 1)];
+  if (most <= 4) {
+    p0 = p1 = make_uint4(0, 0, 0, 0);
+    uint8_t* o = reinterpret_cast<uint8_t*>(stage);
+    for (uint32_t b = bits; b; b &= b - 1) {
+      const int j = __ffs(b) - 1;
+      o[16 * stage_piece(2 * lane + (j >> 4)) + (j & 15)] = sh.in[rank++];
+    }
+    return;
+  }
+  const uint32_t* in32 = reinterpret_cast<const uint32_t*>(sh.in);
+  int at = rank >> 2, shift = (rank & 3) * 8;
+  uint32_t lo = in32[at], hi = in32[at + 1], w[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const uint32_t e = sh.expand[(bits >> (4 * q)) & 15u];
+    w[q] = __byte_perm(__funnelshift_r(lo, hi, shift), 0u, e);
+    shift += e >> 16;
+    if (shift >= 32) {  // at most one word per four kept bytes
+      shift -= 32;
+      lo = hi;
+      hi = in32[++at + 1];
+    }
+  }
+  p0 = make_uint4(w[0], w[1], w[2], w[3]);
+  p1 = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
 // Chunk holding byte `off` of the plane buffer (host placement: level 3's 32
 // planes first, each plane cut into 16 KiB chunks; chunk ids follow the
 // bytes).  Offsets past the buffer map past the last chunk.
-__device__ __forceinline__ int64_t chunk_of_byte(const Geometry& g, int64_t off) {
+__host__ __device__ __forceinline__ int64_t chunk_of_byte(const Geometry& g, int64_t off) {
   int64_t hb = 0, cb = 0;
   for (int l = 3; l >= 0; --l) {
     const int64_t span = g.hastride[l] << 5;
@@ -474,40 +605,126 @@ __device__ __forceinline__ int64_t chunk_of_byte(const Geometry& g, int64_t off)
   return 0;
 }
 
-// Grid-stride over the chunks a decode must visit.  begin/end (device, may
+// Host placement of a byte of the plane buffer: its chunk, the chunk's level,
+// plane and byte range.  The byte is given with the level and plane whose
+// device placement it was computed from; the two placements drift apart by a
+// few bytes per plane, so the chunk is that plane's or a near one's and the
+// walk below takes a step or none (no division).
+struct HostChunk {
+  int64_t id, begin, end;
+  int level, plane;
+};
+__host__ __device__ __forceinline__ int64_t host_stride(const Geometry& g, int l) {
+  return l == 0 ? g.hastride[0] : (l == 1 ? g.hastride[1] : (l == 2 ? g.hastride[2] : g.hastride[3]));
+}
+__host__ __device__ __forceinline__ HostChunk chunk_near(const Geometry& g, int level, int plane, int64_t off) {
+  const int64_t h3 = g.hastride[3] << 5, h2 = h3 + (g.hastride[2] << 5), h1 = h2 + (g.hastride[1] << 5);
+  int l = level, p = plane;
+  int64_t stride = host_stride(g, l);
+  int64_t base = (l == 3 ? 0 : (l == 2 ? h3 : (l == 1 ? h2 : h1))) + p * stride;
+  while (off < base) {
+    if (p == 0) {
+      p = 31;
+      stride = host_stride(g, ++l);
+    } else {
+      --p;
+    }
+    base -= stride;
+  }
+  while (off >= base + stride && !(l == 0 && p == 31)) {
+    base += stride;
+    if (p == 31) {
+      p = 0;
+      stride = host_stride(g, --l);
+    } else {
+      ++p;
+    }
+  }
+  const int64_t k = (off - base) >> 14;
+  static_assert(kChunk == 1 << 14, "chunk index by shift");
+  HostChunk c;
+  c.level = l;
+  c.plane = p;
+  c.begin = base + k * kChunk;
+  c.end = c.begin + kChunk < base + stride ? c.begin + kChunk : base + stride;
+  const int64_t c3 = g.chunks_level[3], c2 = c3 + g.chunks_level[2], c1 = c2 + g.chunks_level[1];
+  const int64_t per = (l == 0 ? g.chunks_level[0] : (l == 1 ? g.chunks_level[1] : (l == 2 ? g.chunks_level[2] : c3))) >> 5;
+  c.id = (l == 3 ? 0 : (l == 2 ? c3 : (l == 1 ? c2 : c1))) + p * per + k;
+  return c;
+}
+
+// Which chunks a decode leaves as zeros: the all-zero ones and, when
+// begin/end select planes, those outside [begin, end) of their level.  sizes
+// == null: every chunk holds bytes (a plane buffer that was not decoded here).
+struct ChunkLive {
+  const uint16_t* sizes;
+  const int* begin;
+  const int* end;
+  __device__ __forceinline__ bool dead(const HostChunk& c) const {
+    if (!sizes) return false;
+    const bool zero = __ldg(sizes + c.id) == kZeroChunkBytes;
+    return zero || (begin && (c.plane < begin[3 - c.level] || c.plane >= end[3 - c.level]));
+  }
+};
+
+// Bytes at either end of a dead chunk that the decoder still writes as zeros
+// when its reader skips dead chunks: an inverse-shuffle item reads up to this
+// many consecutive bytes of a plane and skips them only when one dead chunk
+// holds them all.
+constexpr int kDeadEdge = 128;
+
+// Decode the chunks of a stream into the plane buffer.  begin/end (device, may
 // be null) select the chunks of host planes [begin[3-l], end[3-l]) like
-// zbpc_decode_progressive (zbpc.cu:420-423); then per level only one range
-// of chunk ids matters: the selected planes' chunks and the chunks holding
-// the bytes the inverse shuffle reads for those planes at their device
-// placement (which are zeroed where no selected chunk covers them).  Other
-// chunks are never read, so the walk skips them.  Corrupt chunks raise
-// error_flag = 2.  The payload is decoded from its tail: bitmap 4 B -> 32 B
-// -> 256 B -> 2048 B (fill-forward: byte i = kept byte rank(i) - 1, rank the
-// inclusive flag count), then the nonzero bytes are scattered by the
-// zero-elimination bitmap.
-__global__ void __launch_bounds__(kZThreads, 4)
-zbpc_decode_kernel(const uint8_t* __restrict__ stream, uint64_t stream_bytes, const int64_t* __restrict__ offs,
-                   Geometry g, uint8_t* __restrict__ planes, const int* __restrict__ begin,
-                   const int* __restrict__ end, int* __restrict__ error_flag) {
+// zbpc_decode_progressive (zbpc.cu:420-423).  Two passes over one grid:
+//
+// 1. Dead chunks (all-zero or not selected) that the inverse shuffle reaches:
+//    per level one range of chunk ids, the selected planes' chunks and those
+//    holding the bytes the inverse reads for these planes at their device
+//    placement.  A reader that skips dead chunks (ChunkLive) needs zeros only
+//    within kDeadEdge bytes of their ends (EDGES); otherwise all-zero chunks
+//    are written whole and unselected ones where the inverse reads them.  At
+//    common bounds most chunks are all-zero (the leading planes of small
+//    codes), and not moving their 16 KB here and in the inverse shuffle is
+//    most of what this pass saves.
+// 2. The selected coded chunks, from the table, one CTA of 256 threads each.
+//    The payload is decoded from its tail: bitmap 4 B -> 32 B -> 256 B ->
+//    2048 B (fill-forward: byte i = kept byte rank(i) - 1, rank the inclusive
+//    flag count), then every thread expands two words of 32 zero-elimination
+//    flags (expand_word); the bytes leave through shared memory in coalesced
+//    stores.
+//
+// What bounds pass 2 is instruction issue and the chain of barriers, not
+// memory: on a 1000x777x513 float field at ABS 1e-3 (98 K chunks, two thirds
+// of them coded and sparse) 449 us against 1248 us for one pass of 512-thread
+// CTAs over every chunk, 32 predicated byte loads a thread and six barriers
+// more a chunk; on 128^3 floats at REL 1e-4 8.0 against 11.0 us.
+//
+// Corrupt chunks raise error_flag = 2.
+template <bool EDGES>
+__global__ void __launch_bounds__(kDecThreads, kDecCtas)
+zbpc_decode_kernel(const uint8_t* __restrict__ stream, uint64_t stream_bytes, const ChunkTable table, Geometry g,
+                   uint8_t* __restrict__ planes, const int* __restrict__ begin, const int* __restrict__ end,
+                   int* __restrict__ error_flag) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   DecodeShared& sh = *reinterpret_cast<DecodeShared*>(smem_raw);
   __shared__ int64_t range_start[4], range_len[4];
+  __shared__ uint32_t coded_start[4], coded_len[4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t chunks = g.chunks;
   const uint16_t* sizes = reinterpret_cast<const uint16_t*>(stream + 8);
   const uint8_t* data_in = stream + 8 + 2 * chunks;
   if (tid < 4) {
     const int l = tid;
-    int64_t s = 0, e = 0;
+    int64_t s = 0, e = 0, cs = 0, ce = 0;  // ids to visit; ids of the selected planes' chunks
     if (!begin) {
-      e = l == 0 ? chunks : 0;  // a full decode: every chunk, once
+      ce = e = l == 0 ? chunks : 0;  // a full decode: every chunk, once
     } else if (begin[3 - l] < end[3 - l]) {
       const int lo = begin[3 - l], hi = end[3 - l];
       int64_t cb = 0;
       for (int i = 3; i > l; --i) cb += g.chunks_level[i];
       const int64_t cpp = g.chunks_level[l] >> 5;
-      s = cb + lo * cpp;
-      e = cb + hi * cpp;
+      s = cs = cb + lo * cpp;
+      e = ce = cb + hi * cpp;
       const int64_t a = g.daprefix[l] + (int64_t)lo * g.dstride[l], b = g.daprefix[l] + (int64_t)hi * g.dstride[l];
       const int64_t lim = (int64_t)g.aligned_size;
       if (a < b && a < lim) {
@@ -517,85 +734,110 @@ zbpc_decode_kernel(const uint8_t* __restrict__ stream, uint64_t stream_bytes, co
       }
       s = s < 0 ? 0 : (s > chunks ? chunks : s);
       e = e < s ? s : (e > chunks ? chunks : e);
+      cs = cs < 0 ? 0 : (cs > chunks ? chunks : cs);
+      ce = ce < cs ? cs : (ce > chunks ? chunks : ce);
     }
     range_start[l] = s;
     range_len[l] = e - s;
+    coded_start[l] = table.rank[cs];
+    coded_len[l] = table.rank[ce] - table.rank[cs];
+  }
+  if (tid < 16) {  // nibble of flags -> byte-permute selector (4 = a zero byte) and 8 x kept bytes
+    uint32_t sel = 0, kept = 0;
+    for (int j = 0; j < 4; ++j) {
+      sel |= (((tid >> j) & 1) ? kept : 4u) << (4 * j);
+      kept += (tid >> j) & 1;
+    }
+    sh.expand[tid] = sel | (8 * kept) << 16;
   }
   __syncthreads();
+
+  // ---- dead chunks: a lane classifies one, the warp writes the zeros ----
   const int64_t visits = range_len[0] + range_len[1] + range_len[2] + range_len[3];
-  for (int64_t v = blockIdx.x; v < visits; v += gridDim.x) {
+  const int64_t warps = (int64_t)gridDim.x * kDecWarps;
+  for (int64_t v0 = ((int64_t)blockIdx.x * kDecWarps + warp) * 32; v0 < visits; v0 += warps * 32) {
+    const int64_t v = v0 + lane;
     int64_t id = v;
-    int r = 0;
-    while (r < 3 && id >= range_len[r]) id -= range_len[r++];
-    id += range_start[r];
-    const ChunkLoc loc = locate_chunk(g, id);
-    if (begin) {
-      int64_t cpp = g.chunks_level[loc.level] >> 5;
-      int64_t real = loc.plane * cpp + loc.offset;
-      if (real < begin[3 - loc.level] * cpp || real >= end[3 - loc.level] * cpp) {
-        // A plane this step does not load reads as zero where the inverse
-        // shuffle reads it: the inverse reads, per level l, the planes
-        // [lo, hi) it selects at their device placement, bytes
-        // [daprefix[l] + lo dstride[l], daprefix[l] + hi dstride[l]), which
-        // can reach into the host placement of neighbouring planes.  Only the
-        // part of this chunk inside those ranges is zeroed (all bounds are
-        // multiples of 8); the rest is never read.
-        const int64_t cb = loc.base, ce = loc.base + loc.osize;
+    bool zero = false, unselected = false;
+    int64_t cb = 0, ce = 0;
+    if (v < visits) {
+      int r = 0;
+      while (r < 3 && id >= range_len[r]) id -= range_len[r++];
+      id += range_start[r];
+      const ChunkLoc loc = locate_chunk(g, id);
+      cb = loc.base;
+      ce = cb + loc.osize;
+      if (begin) unselected = loc.plane < begin[3 - loc.level] || loc.plane >= end[3 - loc.level];
+      if (!unselected && sizes[id] == kZeroChunkBytes) {
+        const uint64_t at = (uint64_t)(8 + 2 * chunks + table.offs[id]);
+        const uint8_t* src = data_in + table.offs[id];
+        if (at + kZeroChunkBytes > stream_bytes || (src[0] | (src[1] << 8)) != loc.osize) atomicExch(error_flag, 2);
+        else zero = true;
+      }
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, zero || unselected); todo; todo &= todo - 1) {
+      const int from = __ffs(todo) - 1;
+      const int64_t b = __shfl_sync(0xffffffffu, cb, from), e = __shfl_sync(0xffffffffu, ce, from);
+      const bool all = __shfl_sync(0xffffffffu, (int)zero, from) != 0;
+      auto clear = [&](int64_t a, int64_t z) {  // [a, z), multiples of 8
+        for (int64_t o = a + 8 * lane; o < z; o += 8 * 32) *reinterpret_cast<uint2*>(planes + o) = make_uint2(0, 0);
+      };
+      if constexpr (EDGES) {
+        // kDeadEdge bytes at each end: 16 lanes of 8 bytes each
+        const int64_t o = lane < 16 ? b + 8 * lane : e - kDeadEdge + 8 * (lane - 16);
+        if (o >= b && o < e) *reinterpret_cast<uint2*>(planes + o) = make_uint2(0, 0);
+        static_assert(kDeadEdge == 16 * 8, "one 8-byte store per lane");
+      } else if (all) {
+        clear(b, e);
+      } else {
+        // the inverse reads, per level l, the planes [lo, hi) it selects at
+        // their device placement, bytes [daprefix[l] + lo dstride[l],
+        // daprefix[l] + hi dstride[l]) (multiples of 8); the rest of this
+        // chunk is never read
 #pragma unroll 1
         for (int l = 0; l < 4; ++l) {
           const int lo = begin[3 - l], hi = end[3 - l];
           if (lo >= hi) continue;
           const int64_t r0 = g.daprefix[l] + (int64_t)lo * g.dstride[l], r1 = g.daprefix[l] + (int64_t)hi * g.dstride[l];
-          const int64_t a = cb > r0 ? cb : r0, e = ce < r1 ? ce : r1;
-          for (int64_t o = a + 8 * (int64_t)tid; o < e; o += 8 * (int64_t)kZThreads)
-            *reinterpret_cast<uint2*>(planes + o) = make_uint2(0, 0);
+          clear(b > r0 ? b : r0, e < r1 ? e : r1);
         }
-        continue;
       }
     }
-    const int osize = loc.osize;
-    const int csize = sizes[id];
-    const uint64_t at = (uint64_t)(8 + 2 * chunks + offs[id]);
-    if (csize > osize || at + (uint64_t)csize > stream_bytes) {  // corrupt size table
+  }
+
+  // ---- coded chunks ----
+  const uint32_t coded = coded_len[0] + coded_len[1] + coded_len[2] + coded_len[3];
+  auto entry = [&](uint32_t v) {
+    int r = 0;
+    while (r < 3 && v >= coded_len[r]) v -= coded_len[r++];
+    return table.coded[coded_start[r] + v];
+  };
+  ulonglong2 next = make_ulonglong2(0, 0);
+  if (blockIdx.x < coded) next = entry(blockIdx.x);
+  for (uint32_t v = blockIdx.x; v < coded; v += gridDim.x) {
+    const uint64_t off = next.x & kCodedMask;
+    const int csize = (int)(next.x >> 48), osize = (int)(next.y >> 48);
+    uint8_t* dst = planes + (next.y & kCodedMask);
+    if (v + gridDim.x < coded) next = entry(v + gridDim.x);  // arrives meanwhile
+    if (csize > osize || (uint64_t)(8 + 2 * chunks) + off + (uint64_t)csize > stream_bytes) {  // corrupt size table
       if (tid == 0) atomicExch(error_flag, 2);
       continue;
     }
-    const uint8_t* src = data_in + offs[id];
-    uint8_t* dst = planes + loc.base;
-    const int b0 = tid * 32;
-    if (csize == osize) {  // raw chunk: 32 bytes per thread through shared memory
-      copy_in(sh.in, src, osize);
-      __syncthreads();
-      if (b0 < osize) {
-        const uint2* s2 = reinterpret_cast<const uint2*>(sh.in + b0);
-        uint2* d2 = reinterpret_cast<uint2*>(dst + b0);
-        const int nq = min(4, (osize - b0) >> 3);
-        for (int q = 0; q < nq; ++q) d2[q] = s2[q];
-      }
-      __syncthreads();
+    const uint8_t* src = data_in + off;
+    if (csize == osize) {  // raw chunk (osize is a multiple of 8)
+      copy_words(reinterpret_cast<uint32_t*>(dst), src, osize);
       continue;
     }
-    copy_in(sh.in, src, csize);
+    __syncthreads();  // the previous chunk's payload is no longer read
+    copy_words(reinterpret_cast<uint32_t*>(sh.in), src, csize);
     if (tid == 0) sh.flag = 0;
     __syncthreads();
-    bool bad = csize < 2 || (sh.in[csize - 2] | (sh.in[csize - 1] << 8)) != osize;
-    if (!bad && csize == 2) {  // all zero
-      if (b0 < osize) {
-        uint2* d2 = reinterpret_cast<uint2*>(dst + b0);
-        const int nq = min(4, (osize - b0) >> 3);
-        for (int q = 0; q < nq; ++q) d2[q] = make_uint2(0, 0);
-      }
-      __syncthreads();
-      continue;
-    }
-    if (!bad && csize < 6) bad = true;
-    if (bad) {
+    if (csize < 6 || (sh.in[csize - 2] | (sh.in[csize - 1] << 8)) != osize) {
       if (tid == 0) atomicExch(error_flag, 2);
-      __syncthreads();
       continue;
     }
     // ---- warp 0: bm3 (4 B) -> bm2 (32 B) -> bm1 (256 B) ----
-    int rpos = csize - 6;  // start of bm3
+    const int rpos = csize - 6;  // start of bm3
     if (warp == 0) {
       const uint32_t bm3 = (uint32_t)sh.in[rpos] | ((uint32_t)sh.in[rpos + 1] << 8) |
                            ((uint32_t)sh.in[rpos + 2] << 16) | ((uint32_t)sh.in[rpos + 3] << 24);
@@ -605,7 +847,6 @@ zbpc_decode_kernel(const uint8_t* __restrict__ stream, uint64_t stream_bytes, co
       const int rank3 = __popc(bm3 & (0xffffffffu >> (31 - lane)));
       uint32_t b2 = 0;
       if (p3 >= 0 && rank3 > 0) b2 = sh.in[p3 + rank3 - 1];
-      sh.bm2[lane] = (uint8_t)b2;
       // bm2 flags 256 bits: lane l owns flags 8l..8l+7 = byte b2 of lane l
       const int cnt2 = __popc(b2);
       const int incl2 = warp_incl_scan(cnt2, lane);
@@ -618,56 +859,63 @@ zbpc_decode_kernel(const uint8_t* __restrict__ stream, uint64_t stream_bytes, co
         sh.bm1[8 * lane + k] = (p2 >= 0 && r > 0) ? sh.in[p2 + r - 1] : 0;
       }
       if (lane == 0) {
-        sh.scratch[36] = p2;
+        sh.p2 = p2;
         if (p3 < 0 || p2 < 0) sh.flag = 1;
       }
     }
     __syncthreads();
-    const int p2 = sh.scratch[36];
     if (sh.flag) {
       if (tid == 0) atomicExch(error_flag, 2);
-      __syncthreads();
       continue;
     }
-    // ---- all threads: bm1 (2048 flags) -> bm0 (2048 B); thread t owns bm0 bytes 4t..4t+3 ----
-    const uint32_t f1 = (sh.bm1[tid >> 1] >> (4 * (tid & 1))) & 0xFu;
-    int c1;
-    int r1 = block_excl_scan(__popc(f1), sh.scratch, &c1);
-    const int p1 = p2 - c1;  // RE1 bytes
+    // ---- all threads: bm1 (2048 flags) -> the words first and first + 32 of
+    // the 512-word bitmap, four flags (bitmap bytes) each ----
+    const int first = 64 * warp + lane;
+    const uint32_t fa = (sh.bm1[first >> 1] >> (4 * (first & 1))) & 0xFu;
+    const uint32_t fb = (sh.bm1[(first >> 1) + 16] >> (4 * (first & 1))) & 0xFu;
+    const TwoRanks r1 = block_two_ranks(__popc(fa) | __popc(fb) << 16, sh.scan1);
+    const int p1 = sh.p2 - r1.total;  // RE1 bytes
     if (p1 < 0) {
       if (tid == 0) atomicExch(error_flag, 2);
-      __syncthreads();
       continue;
     }
     // fill-forward: byte i = RE1 byte (rank(i) - 1), rank inclusive; rank 0 -> 0
-    uint32_t bits = 0;
+    auto word_of = [&](uint32_t f, int r) {
+      uint32_t b = 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      r1 += (f1 >> k) & 1u;
-      bits |= (uint32_t)(r1 > 0 ? sh.in[p1 + r1 - 1] : 0) << (8 * k);
-    }
-    // bits = this thread's 32 zero-elimination flags (bytes b0 .. b0+31)
-    int nz;
-    int rank = block_excl_scan(__popc(bits), sh.scratch, &nz);
-    if (b0 < osize) {
-      uint32_t w[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        uint32_t v = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int bit = q * 4 + j;
-          if ((bits >> bit) & 1u) v |= (uint32_t)sh.in[rank] << (8 * j);
-          rank += (bits >> bit) & 1u;
-        }
-        w[q] = v;
+      for (int k = 0; k < 4; ++k) {
+        r += (f >> k) & 1u;
+        b |= (uint32_t)(r > 0 ? sh.in[p1 + r - 1] : 0) << (8 * k);
       }
-      uint2* d2 = reinterpret_cast<uint2*>(dst + b0);
-      const int nq = min(4, (osize - b0) >> 3);
-      for (int q = 0; q < nq; ++q) d2[q] = make_uint2(w[2 * q], w[2 * q + 1]);
+      return b;
+    };
+    const uint32_t ba = word_of(fa, r1.first), bb = word_of(fb, r1.second);
+    const TwoRanks nz = block_two_ranks(__popc(ba) | __popc(bb) << 16, sh.scan2);
+    if (nz.total > p1) {
+      if (tid == 0) atomicExch(error_flag, 2);
+      continue;
     }
-    if (nz > p1 && tid == 0) atomicExch(error_flag, 2);
-    __syncthreads();
+    uint4* stage = sh.out[warp];
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+      const uint32_t bits = half ? bb : ba;
+      const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)__popc(bits));
+      const int b0 = 2048 * warp + 1024 * half;  // the warp's bytes of this half
+      if (b0 >= osize) break;
+      uint2* d2 = reinterpret_cast<uint2*>(dst + b0);
+      if (most > 0) {
+        expand_word(sh, stage, bits, half ? nz.second : nz.first, most);
+        __syncwarp();
+      }
+      const uint2* o2 = reinterpret_cast<const uint2*>(stage);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = 32 * q + lane;
+        const uint2 x = most > 0 ? o2[2 * stage_piece(i >> 1) + (i & 1)] : make_uint2(0, 0);
+        if (b0 + 8 * i < osize) d2[i] = x;
+      }
+      __syncwarp();
+    }
   }
 }
 
