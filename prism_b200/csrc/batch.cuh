@@ -6,12 +6,11 @@
 // of the batch.  Work items of a stage are numbered across the fields (a
 // field's items follow the previous field's), and a kernel maps an item to
 // its field by a binary search over the per-field item prefix.  The predictor
-// and the lossless encoder are persistent kernels whose CTAs pull items from
-// a device counter, so large and small fields share the GPU without a wave
-// tail per field.  Every field's bytes are exactly those of the per-field
-// pipeline: the same tile, shuffle and chunk code runs on each item; the
-// look-back of the encoder ends at the field's first chunk because each field
-// has its own status slice.
+// is a persistent kernel whose CTAs pull items from a device counter (or one
+// CTA per tile) and the lossless encoder strides over the items, so large and
+// small fields share the GPU without a wave tail per field.  Every field's
+// bytes are exactly those of the per-field pipeline: the same tile, shuffle
+// and chunk code runs on each item.
 #pragma once
 #include "autotune.cuh"
 #include "bitplane.cuh"
@@ -41,7 +40,8 @@ struct BatchField {
   int32_t* qc;
   uint8_t* planes;
   void* anchors;
-  unsigned long long* status;
+  int64_t* offs;  // payload offset per chunk
+  uint32_t* rows;  // nonzero planes per shuffle item
   BatchState* st;
   int mode, nb, tsize, pad;
   double bound, alpha;
@@ -263,20 +263,7 @@ __global__ void batch_leftover_kernel(const BatchField* __restrict__ fields, con
   for (int r = blockIdx.x; r < nranges; r += gridDim.x) {
     const BatchRange br = ranges[r];
     const BatchField& f = fields[br.field];
-    const Geometry& g = f.g;
-    for (uint64_t o = threadIdx.x; o < br.len; o += blockDim.x) {
-      const uint64_t b = br.start + o;
-      const uint64_t i = b >> 2;
-      uint8_t v = 0;
-      if (i < g.n) {
-        const uint64_t x = i % g.nx, y = (i / g.nx) % g.ny, z = i / ((uint64_t)g.nx * g.ny);
-        if ((x & 15) | (y & 15) | (z & 15)) {
-          const uint32_t code = (uint32_t)f.qc[level_major_index(g, x, y, z)];
-          v = (uint8_t)(code >> (8 * (b & 3)));
-        }
-      }
-      f.planes[b] = v;
-    }
+    leftover_fill(f.planes, f.qc, f.g, br.start, br.len);
   }
 }
 
@@ -297,67 +284,64 @@ batch_shuffle_kernel(const BatchField* __restrict__ fields, const uint64_t* __re
   if (item >= items) return;
   const int e = find_field(prefix, n, item);
   const BatchField& f = fields[e];
-  shuffle_item(tile[threadIdx.x >> 5], f.qc + f.g.anchors, f.planes, f.g, f.plan, f.nb, (int64_t)(item - prefix[e]));
+  shuffle_item(tile[threadIdx.x >> 5], f.qc + f.g.anchors, f.planes, f.g, f.plan, f.nb, (int64_t)(item - prefix[e]), f.rows);
 }
 
-// persistent lossless encoder over the chunks of all fields
-__global__ void __launch_bounds__(kZThreads, 4)
-batch_encode_kernel(const BatchField* __restrict__ fields, const uint64_t* __restrict__ prefix, int n,
-                    uint64_t items, unsigned long long* __restrict__ ticket, long long spin_limit) {
+__device__ __forceinline__ EncodeJob batch_job(const BatchField& f) {
+  return EncodeJob{f.planes, f.planes, reinterpret_cast<uint16_t*>(f.out + 8)};
+}
+
+// the lossless encoder's three launches over the chunks of all fields
+// (encode_chunks_kernel, scan_stream_kernel, gather_stream_kernel)
+__global__ void __launch_bounds__(kEncThreads, kEncCtas)
+batch_encode_kernel(const BatchField* __restrict__ fields, const uint64_t* __restrict__ prefix, int n, uint64_t items) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  EncodeShared& sh = *reinterpret_cast<EncodeShared*>(smem_raw);
-  while (true) {
-    if (threadIdx.x == 0) sh.ticket = (long long)atomicAdd(ticket, 1ull);
-    __syncthreads();
-    const uint64_t item = (uint64_t)sh.ticket;
-    if (item >= items) break;
-    const int e = find_field(prefix, n, item);
+  EncodeShared2& sh = *reinterpret_cast<EncodeShared2*>(smem_raw);
+  EncodeItem(&list)[kEncThreads] = *reinterpret_cast<EncodeItem(*)[kEncThreads]>(smem_raw + sizeof(EncodeShared2));
+  encode_items(sh, list, items, [&](uint64_t i, EncodeItem& it) {
+    const int e = find_field(prefix, n, i);
     const BatchField& f = fields[e];
-    encode_chunk(sh, f.planes, f.g, f.out, f.status, (int64_t)(item - prefix[e]), f.st->csbp, &f.st->lossless_size,
-                 &f.st->error_flag, spin_limit);
-  }
+    it.job = batch_job(f);
+    it.id = (uint32_t)(i - prefix[e]);
+    const ChunkLoc loc = locate_chunk(f.g, it.id);
+    it.base = loc.base;
+    it.osize = loc.osize;
+    return !chunk_is_zero(f.rows, f.g, f.plan, loc);
+  });
 }
 
-// one warp per field: stream header and padding (zbpc_finish_kernel)
-__global__ void batch_finish_kernel(const BatchField* __restrict__ fields, int n) {
-  const int e = blockIdx.x;
-  if (e >= n) return;
-  const BatchField& f = fields[e];
-  const uint64_t total = 8 + 2 * (uint64_t)f.g.chunks + f.st->lossless_size;
-  const uint64_t pad = (8 - total % 8) % 8;
-  if (threadIdx.x < pad) f.out[total + threadIdx.x] = 0;
-  if (threadIdx.x == 0) {
-    const long long hdr = (long long)f.g.aligned_size;
-    for (int i = 0; i < 8; ++i) f.out[i] = (uint8_t)(hdr >> (8 * i));
-    f.st->padded_size = total + pad;
-  }
+// CTA entries: a field and one of its scan CTAs
+__global__ void __launch_bounds__(kScanThreads)
+batch_scan_kernel(const BatchField* __restrict__ fields, const BatchLastCta* __restrict__ ctas) {
+  const BatchLastCta c = ctas[blockIdx.x];
+  const BatchField& f = fields[c.field];
+  scan_stream(f.out, f.g, f.offs,
+              StreamTotals{f.st->csbp, &f.st->lossless_size, &f.st->padded_size, &f.st->error_flag}, c.cta);
 }
 
-constexpr uint64_t kBatchTrailerSeg = 1u << 16;  // trailer bytes per item
+__global__ void __launch_bounds__(kEncThreads)
+batch_gather_kernel(const BatchField* __restrict__ fields, const uint64_t* __restrict__ prefix, int n, uint64_t items) {
+  __shared__ GatherItem list[kEncThreads];
+  gather_items(list, items, [&](uint64_t i, GatherItem& it) {
+    const int e = find_field(prefix, n, i);
+    const BatchField& f = fields[e];
+    return gather_chunk(batch_job(f), f.g, f.out, f.offs, (int64_t)(i - prefix[e]), it);
+  });
+}
 
-// trailer (trailer_kernel) in items of kBatchTrailerSeg bytes over the group
+constexpr uint64_t kBatchTrailerSeg = 1u << 12;  // trailer bytes per item
+
+// trailer in items of kBatchTrailerSeg bytes over the group
 template <class T>
 __global__ void batch_trailer_kernel(const BatchField* __restrict__ fields, const int* __restrict__ gidx,
                                      const uint64_t* __restrict__ prefix, int n, uint64_t items) {
   for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
     const int e = find_field(prefix, n, item);
     const BatchField& f = fields[gidx[e]];
-    const PredParams<T>* p = reinterpret_cast<const PredParams<T>*>(f.st->params);
-    uint8_t* tr = f.out + f.st->padded_size;
-    const uint64_t total = 1040 + f.g.anchors * sizeof(T);
-    const uint64_t b0 = (item - prefix[e]) * kBatchTrailerSeg, b1 = min(b0 + kBatchTrailerSeg, total);
-    const uint8_t* range = reinterpret_cast<const uint8_t*>(&f.st->range);
-    const uint8_t* csbp = reinterpret_cast<const uint8_t*>(f.st->csbp);
-    const uint8_t* anchors = reinterpret_cast<const uint8_t*>(f.anchors);
-    for (uint64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
-      uint8_t v;
-      if (i < 4) v = p->use_md[i];
-      else if (i < 8) v = p->reverse[i - 4];
-      else if (i < 16) v = range[i - 8];
-      else if (i < 1040) v = csbp[i - 16];
-      else v = anchors[i - 1040];
-      tr[i] = v;
-    }
+    const uint64_t w0 = (item - prefix[e]) * (kBatchTrailerSeg / 4);
+    write_trailer(f.out + f.st->padded_size, reinterpret_cast<const PredParams<T>*>(f.st->params), &f.st->range,
+                  f.st->csbp, reinterpret_cast<const T*>(f.anchors), f.g.anchors, w0 + threadIdx.x, blockDim.x,
+                  w0 + kBatchTrailerSeg / 4);
   }
 }
 

@@ -16,9 +16,7 @@ struct prism_batch {
   unsigned char* dev = nullptr;  // one allocation for all device state
   BatchField* d_fields = nullptr;
   BatchState* d_states = nullptr;
-  unsigned long long* d_status = nullptr;
-  size_t status_bytes = 0;
-  unsigned long long* d_counters = nullptr;  // predict f32 x2, f64 x2, encode
+  unsigned long long* d_counters = nullptr;  // predict f32 x2, f64 x2
   BatchResult* d_results = nullptr;
   BatchResult* h_results = nullptr;  // pinned
   struct Group {
@@ -47,6 +45,8 @@ struct prism_batch {
   int npre = 0;
   BatchLastCta* d_post = nullptr;
   int npost = 0;
+  BatchLastCta* d_scan = nullptr;
+  int nscan = 0;
   BatchZero* d_zero = nullptr;
   int nzero = 0;
   int sm_count = 148;
@@ -153,29 +153,15 @@ int enqueue_group_back(prism_batch* b, const prism_batch::Group& gr, cudaStream_
 
 int enqueue_encode(prism_batch* b, int ctas, cudaStream_t st, uint64_t& launches) {
   unsigned grid = (unsigned)std::min<uint64_t>(b->chunk_items, (uint64_t)b->sm_count * ctas);
-  batch_encode_kernel<<<grid, kZThreads, sizeof(EncodeShared), st>>>(b->d_fields, b->d_chunk_prefix, b->n,
-                                                                     b->chunk_items, b->d_counters + 4,
-                                                                     (long long)1 << 22);
+  batch_encode_kernel<<<grid, kEncThreads, encode_smem_bytes(), st>>>(b->d_fields, b->d_chunk_prefix, b->n,
+                                                                      b->chunk_items);
   ++launches;
   BCK(cudaGetLastError());
   return PRISM_OK;
 }
 
-// The whole pipeline on stream st (what the graph holds).
-int enqueue_all(prism_batch* b, cudaStream_t st, uint64_t& launches) {
-  launches = 0;
-  BCK(cudaMemsetAsync(b->d_states, 0, sizeof(BatchState) * b->n, st));
-  BCK(cudaMemsetAsync(b->d_status, 0, b->status_bytes, st));
-  BCK(cudaMemsetAsync(b->d_counters, 0, 8 * sizeof(unsigned long long), st));
-  int rc;
-  if ((rc = enqueue_group_front<float>(b, b->grp[0], st, launches))) return rc;
-  if ((rc = enqueue_group_front<double>(b, b->grp[1], st, launches))) return rc;
-  if (b->nzero) {
-    batch_zero_kernel<<<std::min(b->nzero, 4096), 256, 0, st>>>(b->d_zero, b->nzero);
-    ++launches;
-  }
-  if ((rc = enqueue_group_predict<float>(b, b->grp[0], 0, b->pred_ctas[0], st, launches))) return rc;
-  if ((rc = enqueue_group_predict<double>(b, b->grp[1], 1, b->pred_ctas[1], st, launches))) return rc;
+// leftover bytes, last shuffle blocks and bulk shuffle
+int enqueue_shuffle(prism_batch* b, cudaStream_t st, uint64_t& launches) {
   if (b->nranges) {
     batch_leftover_kernel<<<std::min(b->nranges, 4096), 256, 0, st>>>(b->d_fields, b->d_ranges, b->nranges);
     ++launches;
@@ -193,9 +179,30 @@ int enqueue_all(prism_batch* b, cudaStream_t st, uint64_t& launches) {
     batch_last_block_kernel<<<b->npost, 512, 0, st>>>(b->d_fields, b->d_post);
     ++launches;
   }
+  BCK(cudaGetLastError());
+  return PRISM_OK;
+}
+
+// The whole pipeline on stream st (what the graph holds).
+int enqueue_all(prism_batch* b, cudaStream_t st, uint64_t& launches) {
+  launches = 0;
+  BCK(cudaMemsetAsync(b->d_states, 0, sizeof(BatchState) * b->n, st));
+  BCK(cudaMemsetAsync(b->d_counters, 0, 8 * sizeof(unsigned long long), st));
+  int rc;
+  if ((rc = enqueue_group_front<float>(b, b->grp[0], st, launches))) return rc;
+  if ((rc = enqueue_group_front<double>(b, b->grp[1], st, launches))) return rc;
+  if (b->nzero) {
+    batch_zero_kernel<<<std::min(b->nzero, 4096), 256, 0, st>>>(b->d_zero, b->nzero);
+    ++launches;
+  }
+  if ((rc = enqueue_group_predict<float>(b, b->grp[0], 0, b->pred_ctas[0], st, launches))) return rc;
+  if ((rc = enqueue_group_predict<double>(b, b->grp[1], 1, b->pred_ctas[1], st, launches))) return rc;
+  if ((rc = enqueue_shuffle(b, st, launches))) return rc;
   if ((rc = enqueue_encode(b, b->enc_ctas, st, launches))) return rc;
-  batch_finish_kernel<<<b->n, 32, 0, st>>>(b->d_fields, b->n);
-  ++launches;
+  batch_scan_kernel<<<b->nscan, kScanThreads, 0, st>>>(b->d_fields, b->d_scan);
+  batch_gather_kernel<<<(unsigned)std::min<uint64_t>(b->chunk_items, (uint64_t)b->sm_count * 8), kEncThreads, 0, st>>>(
+      b->d_fields, b->d_chunk_prefix, b->n, b->chunk_items);
+  launches += 2;
   if ((rc = enqueue_group_back<float>(b, b->grp[0], st, launches))) return rc;
   if ((rc = enqueue_group_back<double>(b, b->grp[1], st, launches))) return rc;
   BCK(cudaMemcpyAsync(b->h_results, b->d_results, sizeof(BatchResult) * b->n, cudaMemcpyDeviceToHost, st));
@@ -203,15 +210,18 @@ int enqueue_all(prism_batch* b, cudaStream_t st, uint64_t& launches) {
   return PRISM_OK;
 }
 
-// Time `fn` (which enqueues on st) over two runs; the faster one counts.
-template <class Fn>
-int time_stage(prism_batch* b, cudaStream_t st, Fn fn, double* ms) {
+// Time `fn` (which enqueues on st) over two runs, `prepare` enqueued before
+// each and not timed; the faster one counts.
+template <class Pre, class Fn>
+int time_stage(prism_batch* b, cudaStream_t st, Pre prepare, Fn fn, double* ms) {
   cudaEvent_t e0, e1;
   BCK(cudaEventCreate(&e0));
   BCK(cudaEventCreate(&e1));
   double best = 1e30;
   int rc = PRISM_OK;
   for (int r = 0; r < 2 && rc == PRISM_OK; ++r) {
+    rc = prepare();
+    if (rc) break;
     cudaEventRecord(e0, st);
     rc = fn();
     cudaEventRecord(e1, st);
@@ -240,7 +250,7 @@ int tune_schedule(prism_batch* b, cudaStream_t st) {
     int pick = b->pred_max[g];
     for (int c = 0; c <= b->pred_max[g]; ++c) {  // 0: one CTA per tile
       double ms = 0;
-      rc = time_stage(b, st, [&]() -> int {
+      rc = time_stage(b, st, []() -> int { return PRISM_OK; }, [&]() -> int {
         cudaMemsetAsync(b->d_counters + 2 * g, 0, 2 * sizeof(unsigned long long), st);
         uint64_t l = 0;
         return g == 0 ? enqueue_group_predict<float>(b, b->grp[0], 0, c, st, l)
@@ -256,12 +266,9 @@ int tune_schedule(prism_batch* b, cudaStream_t st) {
   int pick = b->enc_max;
   for (int c = 1; c <= b->enc_max; ++c) {
     double ms = 0;
-    rc = time_stage(b, st, [&]() -> int {
-      cudaMemsetAsync(b->d_status, 0, b->status_bytes, st);
-      cudaMemsetAsync(b->d_counters + 4, 0, sizeof(unsigned long long), st);
-      uint64_t l = 0;
-      return enqueue_encode(b, c, st, l);
-    }, &ms);
+    uint64_t l = 0;  // the encoder works in place: shuffle again before each run
+    rc = time_stage(b, st, [&]() -> int { return enqueue_shuffle(b, st, l); },
+                    [&]() -> int { return enqueue_encode(b, c, st, l); }, &ms);
     if (rc) return rc;
     if (ms < best) { best = ms; pick = c; }
   }
@@ -288,7 +295,7 @@ int batch_plan(prism_batch* b) {
   std::vector<BatchField> fields(n);
   std::vector<uint64_t> shuf_prefix(n + 1, 0), chunk_prefix(n + 1, 0);
   std::vector<BatchRange> ranges;
-  std::vector<BatchLastCta> pre, post;
+  std::vector<BatchLastCta> pre, post, scan;
   std::vector<std::pair<size_t, uint64_t>> zero_rel;  // (field qc offset in ints, len) resolved later
   struct GroupHost {
     std::vector<int> idx;
@@ -296,8 +303,8 @@ int batch_plan(prism_batch* b) {
     std::vector<BatchWindow> wins;
   } gh[2];
   Carve cv;
-  std::vector<size_t> off_qc(n), off_planes(n), off_anchors(n), off_status(n);
-  size_t status_total = 0;
+  std::vector<size_t> off_qc(n), off_planes(n), off_anchors(n), off_chunk(n), off_rows(n);
+  size_t chunk_total = 0;
   for (int i = 0; i < n; ++i) {
     const prism_field_desc& d = b->desc[i];
     const Geometry& g = b->geo[i];
@@ -315,8 +322,11 @@ int batch_plan(prism_batch* b) {
     off_qc[i] = cv.take<int32_t>(qc_len(g));
     off_planes[i] = cv.take<uint8_t>(g.aligned_size + 64);
     off_anchors[i] = cv.take<double>(g.anchors);
-    off_status[i] = status_total;
-    status_total += (size_t)g.chunks;
+    off_rows[i] = cv.take<uint32_t>((size_t)f.plan.items + 4);
+    off_chunk[i] = chunk_total;
+    chunk_total += (size_t)g.chunks;
+    const int scans = (int)((g.chunks + kScanItems - 1) / kScanItems);
+    for (int c = 0; c < scans; ++c) scan.push_back(BatchLastCta{i, c, scans, 0});
     // work items
     shuf_prefix[i + 1] = shuf_prefix[i] + (uint64_t)f.plan.items;
     chunk_prefix[i + 1] = chunk_prefix[i] + (uint64_t)g.chunks;
@@ -349,12 +359,13 @@ int batch_plan(prism_batch* b) {
   }
   // ---- device layout ----
   size_t o_fields = cv.take<BatchField>(n), o_states = cv.take<BatchState>(n);
-  size_t o_status = cv.take<unsigned long long>(std::max<size_t>(status_total, 1));
+  size_t o_offs = cv.take<int64_t>(std::max<size_t>(chunk_total, 1));
   size_t o_counters = cv.take<unsigned long long>(8), o_results = cv.take<BatchResult>(n);
   size_t o_shuf = cv.take<uint64_t>(n + 1), o_chunk = cv.take<uint64_t>(n + 1);
   size_t o_ranges = cv.take<BatchRange>(std::max<size_t>(ranges.size(), 1));
   size_t o_pre = cv.take<BatchLastCta>(std::max<size_t>(pre.size(), 1));
   size_t o_post = cv.take<BatchLastCta>(std::max<size_t>(post.size(), 1));
+  size_t o_scan = cv.take<BatchLastCta>(std::max<size_t>(scan.size(), 1));
   size_t o_zero = cv.take<BatchZero>(std::max<size_t>(zero_rel.size(), 1));
   struct GroupOff { size_t idx, ext, extpart, win, wins, partial, t0, t1, tr; } go[2];
   for (int k = 0; k < 2; ++k) {
@@ -380,15 +391,14 @@ int batch_plan(prism_batch* b) {
     fields[i].qc = reinterpret_cast<int32_t*>(base + off_qc[i]);
     fields[i].planes = base + off_planes[i];
     fields[i].anchors = base + off_anchors[i];
-    fields[i].status = reinterpret_cast<unsigned long long*>(base + o_status) + off_status[i];
+    fields[i].offs = reinterpret_cast<int64_t*>(base + o_offs) + off_chunk[i];
+    fields[i].rows = reinterpret_cast<uint32_t*>(base + off_rows[i]);
     fields[i].st = reinterpret_cast<BatchState*>(base + o_states) + i;
   }
   std::vector<BatchZero> zeros;
   for (auto& z : zero_rel) zeros.push_back(BatchZero{reinterpret_cast<int32_t*>(base) + z.first, z.second});
   b->d_fields = reinterpret_cast<BatchField*>(base + o_fields);
   b->d_states = reinterpret_cast<BatchState*>(base + o_states);
-  b->d_status = reinterpret_cast<unsigned long long*>(base + o_status);
-  b->status_bytes = std::max<size_t>(status_total, 1) * sizeof(unsigned long long);
   b->d_counters = reinterpret_cast<unsigned long long*>(base + o_counters);
   b->d_results = reinterpret_cast<BatchResult*>(base + o_results);
   b->d_shuf_prefix = reinterpret_cast<uint64_t*>(base + o_shuf);
@@ -396,6 +406,8 @@ int batch_plan(prism_batch* b) {
   b->d_ranges = reinterpret_cast<BatchRange*>(base + o_ranges);
   b->d_pre = reinterpret_cast<BatchLastCta*>(base + o_pre);
   b->d_post = reinterpret_cast<BatchLastCta*>(base + o_post);
+  b->d_scan = reinterpret_cast<BatchLastCta*>(base + o_scan);
+  b->nscan = (int)scan.size();
   b->d_zero = reinterpret_cast<BatchZero*>(base + o_zero);
   b->shuf_items = shuf_prefix[n];
   b->chunk_items = chunk_prefix[n];
@@ -412,6 +424,7 @@ int batch_plan(prism_batch* b) {
   BCK(up(b->d_ranges, ranges.data(), sizeof(BatchRange) * ranges.size()));
   BCK(up(b->d_pre, pre.data(), sizeof(BatchLastCta) * pre.size()));
   BCK(up(b->d_post, post.data(), sizeof(BatchLastCta) * post.size()));
+  BCK(up(b->d_scan, scan.data(), sizeof(BatchLastCta) * scan.size()));
   BCK(up(b->d_zero, zeros.data(), sizeof(BatchZero) * zeros.size()));
   for (int k = 0; k < 2; ++k) {
     GroupHost& G = gh[k];
@@ -464,7 +477,7 @@ int batch_plan(prism_batch* b) {
                                                                  &dummy)))
     return rc;
   b->pred_max[1] = std::min(b->pred_max[1], dummy);
-  if ((rc = max_ctas<batch_encode_kernel>(b, kZThreads, (int)sizeof(EncodeShared), &b->enc_max))) return rc;
+  if ((rc = max_ctas<batch_encode_kernel>(b, kEncThreads, encode_smem_bytes(), &b->enc_max))) return rc;
   b->pred_ctas[0] = b->pred_max[0];
   b->pred_ctas[1] = b->pred_max[1];
   b->enc_ctas = b->enc_max;

@@ -167,7 +167,8 @@ __device__ __forceinline__ void locate_item(const ShufPlan& s, int64_t item, int
   *local = item - (k == 0 ? s.item_prefix[0] : (k == 1 ? s.item_prefix[1] : (k == 2 ? s.item_prefix[2] : s.item_prefix[3])));
 }
 
-// codes (qc + anchors, device code space) -> planes.  A warp takes 1024
+// codes (qc + anchors, device code space) -> planes, and (rows not null) per
+// item the mask of its planes with a nonzero byte.  A warp takes 1024
 // consecutive codes of one level: 32 coalesced 128-byte loads into a padded
 // shared-memory tile, from which lane l takes its 32 consecutive codes
 // 32l..32l+31 (in plane-bit order), one in-register 32x32 bit transpose, and
@@ -176,7 +177,7 @@ __device__ __forceinline__ void locate_item(const ShufPlan& s, int64_t item, int
 // One warp work item of the forward shuffle (tw: the warp's staging tile).
 __device__ __forceinline__ void shuffle_item(uint32_t (&tw)[32][33], const int32_t* __restrict__ codes,
                                              uint8_t* __restrict__ planes, const Geometry& g, const ShufPlan& plan,
-                                             int nb, int64_t item) {
+                                             int nb, int64_t item, uint32_t* rows_out) {
   const int lane = threadIdx.x & 31;
   int level;
   int64_t local;
@@ -187,6 +188,7 @@ __device__ __forceinline__ void shuffle_item(uint32_t (&tw)[32][33], const int32
   const int32_t* src = codes + pick4(plan.seg_start, level) + first;
   // tw[it][j] = transformed code 32 it + j (0 past the end: sign_transform(0)
   // = 0); all 32 loads are issued before the first store
+  uint32_t any = 0;
   {
     int32_t c[32];
 #pragma unroll
@@ -195,7 +197,16 @@ __device__ __forceinline__ void shuffle_item(uint32_t (&tw)[32][33], const int32
       c[it] = idx < count ? __ldg(src + idx) : 0;
     }
 #pragma unroll
-    for (int it = 0; it < 32; ++it) tw[it][lane] = sign_transform(c[it], nb);
+    for (int it = 0; it < 32; ++it) {
+      const uint32_t w = sign_transform(c[it], nb);
+      any |= w;
+      tw[it][lane] = w;
+    }
+  }
+  // bit 31 - p: plane p of the item has a nonzero byte
+  if (rows_out) {
+    const uint32_t rows = __reduce_or_sync(0xffffffffu, any);
+    if (lane == 0) rows_out[item] = rows;
   }
   __syncwarp();
   uint32_t a[32];
@@ -226,11 +237,81 @@ __device__ __forceinline__ void shuffle_item(uint32_t (&tw)[32][33], const int32
 
 __global__ void __launch_bounds__(kShufWarps * 32)
 bitshuffle_kernel(const int32_t* __restrict__ codes, uint8_t* __restrict__ planes, Geometry g,
-                  ShufPlan plan, int nb) {
+                  ShufPlan plan, int nb, uint32_t* rows) {
   __shared__ uint32_t tile[kShufWarps][32][33];
   int64_t item = (int64_t)blockIdx.x * kShufWarps + (threadIdx.x >> 5);
   if (item >= plan.items) return;
-  shuffle_item(tile[threadIdx.x >> 5], codes, planes, g, plan, nb, item);
+  shuffle_item(tile[threadIdx.x >> 5], codes, planes, g, plan, nb, item, rows);
+}
+
+// Whether every byte of host chunk `loc` is known to be zero before it is
+// read: from `rows` (16-byte aligned, null: nothing is known), the bulk
+// shuffle's mask of nonzero planes per item, over the items at the chunk's
+// bytes in the device placement.  Chunks with bytes of the leftover ranges or
+// the last shuffle block (the ends of the planes) are not known; the zero
+// words that block spills past a plane change nothing.  (Per-chunk flags
+// raised by the shuffle instead would be stored to by 128 items a chunk at
+// about the same time; those stores alone took nine times the shuffle.)
+__device__ __forceinline__ bool chunk_is_zero(const uint32_t* __restrict__ rows, const Geometry& g, const ShufPlan& plan,
+                                              const ChunkLoc& loc) {
+  if (!rows) return false;
+  int l = loc.level, p = (int)loc.plane;
+  int64_t stride = pick4(g.dstride, l), start = pick4(g.daprefix, l) + p * stride;
+  auto step = [&](int by) {  // to the next or previous plane
+    if (by > 0) start += stride;
+    p += by;
+    if (p == 32 || p < 0) {
+      l -= by;
+      p = p < 0 ? 31 : 0;
+      stride = pick4(g.dstride, l);
+    }
+    if (by < 0) start -= stride;
+  };
+  while (loc.base < start) step(-1);
+  const int64_t end = loc.base + loc.osize;
+  int64_t at = loc.base;
+  while (at < end) {
+    while (at >= start + stride) {
+      if (l == 0 && p == 31) return false;  // past the device placement: leftover bytes
+      step(1);
+    }
+    const int64_t stop = end < start + stride ? end : start + stride;
+    const int64_t bulk = pick4(plan.proc, l) / 8;  // the plane's bytes of bulk items
+    const int64_t b0 = at - start, b1 = stop - start;
+    if (b1 > bulk) return false;
+    {
+      const int64_t first = l == 3 ? plan.item_prefix[0] : (l == 2 ? plan.item_prefix[1]
+                                                                   : (l == 1 ? plan.item_prefix[2] : plan.item_prefix[3]));
+      const int64_t i0 = first + (b0 >> 7), i1 = first + ((b1 - 1) >> 7) + 1;
+      static_assert(kShufCodes / 8 == 1 << 7, "bytes of a plane per item");
+#pragma unroll 4
+      for (int64_t i = i0 & ~(int64_t)3; i < i1; i += 4) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(rows + i));
+        uint32_t any = (i >= i0 ? v.x : 0u) | (i + 1 >= i0 && i + 1 < i1 ? v.y : 0u) |
+                       (i + 2 >= i0 && i + 2 < i1 ? v.z : 0u) | (i + 3 < i1 ? v.w : 0u);
+        if ((any >> (31 - p)) & 1u) return false;
+      }
+    }
+    at = stop;
+  }
+  return true;
+}
+
+// The chunks of a plane buffer (encode_items), all-zero ones by `rows`
+// (chunk_is_zero).
+__global__ void __launch_bounds__(kEncThreads, kEncCtas)
+encode_chunks_kernel(const EncodeJob job, Geometry g, ShufPlan plan, const uint32_t* __restrict__ rows) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  EncodeShared2& sh = *reinterpret_cast<EncodeShared2*>(smem_raw);
+  EncodeItem(&list)[kEncThreads] = *reinterpret_cast<EncodeItem(*)[kEncThreads]>(smem_raw + sizeof(EncodeShared2));
+  encode_items(sh, list, (uint64_t)g.chunks, [&](uint64_t i, EncodeItem& it) {
+    const ChunkLoc loc = locate_chunk(g, (int64_t)i);
+    it.job = job;
+    it.id = (uint32_t)i;
+    it.base = loc.base;
+    it.osize = loc.osize;
+    return !chunk_is_zero(rows, g, plan, loc);
+  });
 }
 
 // planes -> codes; begin/end (device, may be null) restrict each level to
@@ -532,24 +613,43 @@ struct RangeList {
   ByteRange r[kMaxRanges];
 };
 
-__global__ void leftover_fill_kernel(uint8_t* __restrict__ planes, const int32_t* __restrict__ qc, Geometry g,
-                                     const RangeList ranges, int nranges) {
-  for (int r = blockIdx.x; r < nranges; r += gridDim.x) {
-    ByteRange br = ranges.r[r];
-    for (uint64_t o = threadIdx.x; o < br.len; o += blockDim.x) {
-      uint64_t b = br.start + o;
-      uint64_t i = b >> 2;
-      uint8_t v = 0;
-      if (i < g.n) {
-        uint64_t x = i % g.nx, y = (i / g.nx) % g.ny, z = i / ((uint64_t)g.nx * g.ny);
-        if ((x & 15) | (y & 15) | (z & 15)) {
-          uint32_t code = (uint32_t)qc[level_major_index(g, x, y, z)];
-          v = (uint8_t)(code >> (8 * (b & 3)));
-        }
+// One range by one CTA, a thread per code: the (up to) four bytes of a code
+// come from one slot lookup, in 32-bit arithmetic where the field allows it.
+__device__ __forceinline__ void leftover_fill(uint8_t* __restrict__ planes, const int32_t* __restrict__ qc,
+                                              const Geometry& g, const uint64_t start, const uint64_t len) {
+  const uint64_t w0 = start >> 2, w1 = (start + len + 3) >> 2;
+  const bool small = g.n >> 32 == 0;
+  for (uint64_t i = w0 + threadIdx.x; i < w1; i += blockDim.x) {
+    uint32_t code = 0;
+    if (i < g.n) {
+      uint64_t x, y, z;
+      if (small) {
+        const uint32_t row = (uint32_t)i / g.nx, zz = row / g.ny;
+        x = (uint32_t)i - row * g.nx;
+        y = row - zz * g.ny;
+        z = zz;
+      } else {
+        const uint64_t row = i / g.nx;
+        x = i - row * g.nx;
+        z = row / g.ny;
+        y = row - z * g.ny;
       }
-      planes[b] = v;
+      if ((x & 15) | (y & 15) | (z & 15)) code = (uint32_t)qc[level_major_index(g, x, y, z)];
+    }
+    const uint64_t b = 4 * i;
+    if (b >= start && b + 4 <= start + len) {
+      *reinterpret_cast<uint32_t*>(planes + b) = code;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (b + k >= start && b + k < start + len) planes[b + k] = (uint8_t)(code >> (8 * k));
     }
   }
+}
+
+__global__ void leftover_fill_kernel(uint8_t* __restrict__ planes, const int32_t* __restrict__ qc, Geometry g,
+                                     const RangeList ranges, int nranges) {
+  for (int r = blockIdx.x; r < nranges; r += gridDim.x) leftover_fill(planes, qc, g, ranges.r[r].start, ranges.r[r].len);
 }
 
 // Byte ranges of the plane buffer the bulk shuffle (positions before the

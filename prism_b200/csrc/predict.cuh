@@ -1548,6 +1548,32 @@ reconstruct_kernel(const int32_t* __restrict__ qc, const T* __restrict__ anchors
   }
 }
 
+// Trailer of a container (compress_merge, compressor.cu:139-151): use_md[4],
+// reverse[4], double range, size_t comp_size_bp[4][32], anchors.  Words w,
+// w + step, ... below `limit` (every field is a multiple of 4 bytes); stored
+// as words where the trailer is aligned for it.
+template <class T>
+__device__ __forceinline__ void write_trailer(uint8_t* tr, const PredParams<T>* p, const double* range,
+                                              const uint64_t* csbp, const T* anchors, uint64_t nanchors, uint64_t w,
+                                              uint64_t step, uint64_t limit) {
+  const uint64_t total = (1040 + nanchors * sizeof(T)) / 4;
+  const bool aligned = (reinterpret_cast<uintptr_t>(tr) & 3) == 0;
+  for (; w < total && w < limit; w += step) {
+    uint32_t v;
+    if (w == 0) v = p->use_md[0] | p->use_md[1] << 8 | p->use_md[2] << 16 | (uint32_t)p->use_md[3] << 24;
+    else if (w == 1) v = p->reverse[0] | p->reverse[1] << 8 | p->reverse[2] << 16 | (uint32_t)p->reverse[3] << 24;
+    else if (w < 4) v = reinterpret_cast<const uint32_t*>(range)[w - 2];
+    else if (w < 260) v = reinterpret_cast<const uint32_t*>(csbp)[w - 4];
+    else v = reinterpret_cast<const uint32_t*>(anchors)[w - 260];
+    if (aligned) {
+      reinterpret_cast<uint32_t*>(tr)[w] = v;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) tr[4 * w + k] = (uint8_t)(v >> (8 * k));
+    }
+  }
+}
+
 template <class T>
 constexpr int compress_smem_bytes() { return (int)sizeof(CompressSmem<T>); }
 template <class T>

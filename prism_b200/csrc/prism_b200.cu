@@ -92,7 +92,7 @@ struct ProgMirror {
 };
 
 struct prism_handle {
-  DevBuf qc, planes, status, offs, part, wins, ranges, anchors, small, dev_in, dev_out, zero_anchors;
+  DevBuf qc, planes, marks, offs, part, wins, ranges, anchors, small, dev_in, dev_out, zero_anchors;
   DevBuf qc_odd;  // the code buffer of a progressive object's odd-numbered steps
   DevBuf ext;     // per-CTA partials of the extrema scan
   DevBuf sbatch;  // batched strategy searches: cells, inputs and states
@@ -336,11 +336,17 @@ static int launch_reconstruct(prism_handle* h, const int32_t* qc, const T* ancho
   return PRISM_OK;
 }
 
+// `marks`: an encode's nonzero planes per shuffle item, or the one-launch
+// encoder's status word per chunk
+static size_t marks_bytes(const Geometry& g) {
+  return std::max((size_t)g.chunks * sizeof(unsigned long long), ((size_t)(g.n / kShufCodes) + 16) * sizeof(uint32_t));
+}
+
 static int ensure_common(prism_handle* h, const Geometry& g) {
   ++h->epoch;
   CKA(h->qc.ensure(qc_len(g) * sizeof(int32_t)));
   CKA(h->planes.ensure(g.aligned_size + 64));
-  CKA(h->status.ensure((size_t)g.chunks * sizeof(unsigned long long)));
+  CKA(h->marks.ensure(marks_bytes(g)));
   CKA(h->offs.ensure(chunk_table_bytes(g.chunks)));
   CKA(h->anchors.ensure(g.anchors * 8 + 64));
   CKA(h->small.ensure(sizeof(Small)));
@@ -453,8 +459,9 @@ static int zero_code_padding(prism_handle* h, const Geometry& g, cudaStream_t st
   return PRISM_OK;
 }
 
+// rows (may be null): nonzero planes per shuffle item, for launch_encode
 static int launch_bitshuffle(prism_handle* h, const int32_t* qc, const Geometry& g, int nb, uint8_t* planes,
-                             cudaStream_t st) {
+                             uint32_t* rows, cudaStream_t st) {
   int64_t start_last = (g.sh_grid - 1) * (int64_t)kChunk;
   ShufPlan plan = make_shuf_plan(g, start_last);
   RangeList rng;
@@ -469,7 +476,7 @@ static int launch_bitshuffle(prism_handle* h, const int32_t* qc, const Geometry&
   if (!last_last) shuffle_last_block_kernel<<<shuffle_last_block_grid(g), 512, 0, st>>>(codes, planes, g, nb, g.aligned_size);
   if (plan.items > 0) {
     int64_t blocks = (plan.items + kShufWarps - 1) / kShufWarps;
-    bitshuffle_kernel<<<(unsigned)blocks, kShufWarps * 32, 0, st>>>(codes, planes, g, plan, nb);
+    bitshuffle_kernel<<<(unsigned)blocks, kShufWarps * 32, 0, st>>>(codes, planes, g, plan, nb, rows);
   }
   if (last_last) shuffle_last_block_kernel<<<shuffle_last_block_grid(g), 512, 0, st>>>(codes, planes, g, nb, g.aligned_size);
   prof_end(h, kStShuffle, st);
@@ -504,22 +511,47 @@ static int launch_inverse(prism_handle* h, const uint8_t* planes, const Geometry
   return PRISM_OK;
 }
 
-// first_ticket > 0 leaves the chunks before it unencoded, so the first
-// encoded chunk's look-back never sees its predecessor published: used only by
-// the self-test of the bounded wait (prism_lossless_wait_selftest).
-static int launch_encode(prism_handle* h, const uint8_t* planes, const Geometry& g, uint8_t* stream,
-                         cudaStream_t st, int first_ticket = 0, long long spin_limit = (long long)1 << 22) {
+// Encode a plane buffer to a stream; payloads are staged in `slots` (plane
+// buffer sized; may be `planes`, which is then overwritten).  rows: from
+// launch_bitshuffle of these planes, or null.
+static int launch_encode(prism_handle* h, const uint8_t* planes, uint8_t* slots, const uint32_t* rows,
+                         const Geometry& g, uint8_t* stream, cudaStream_t st) {
   Small* s = small(h);
-  CK(cudaMemsetAsync(h->status.p, 0, (size_t)g.chunks * sizeof(unsigned long long), st));
+  const EncodeJob job{planes, slots, reinterpret_cast<uint16_t*>(stream + 8)};
+  int64_t* offs = h->offs.as<int64_t>();
+  const int smem = encode_smem_bytes();
+  CK(smem_limit<encode_chunks_kernel>(smem));
+  const int blocks = (int)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * kEncCtas);
+  prof_begin(h, kStEncode, st);
+  encode_chunks_kernel<<<blocks, kEncThreads, smem, st>>>(job, g, make_shuf_plan(g, (g.sh_grid - 1) * (int64_t)kChunk),
+                                                           rows);
+  scan_stream_kernel<<<(unsigned)((g.chunks + kScanItems - 1) / kScanItems), kScanThreads, 0, st>>>(
+      stream, g, offs, StreamTotals{s->csbp, &s->lossless_size, &s->padded_size, &s->error_flag});
+  gather_stream_kernel<<<(unsigned)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * 8), kEncThreads, 0, st>>>(
+      job, g, stream, offs);
+  prof_end(h, kStEncode, st);
+  h->launches += 3;
+  CK(cudaGetLastError());
+  return PRISM_OK;
+}
+
+// The one-launch encoder with its tickets starting at first_ticket > 0, so
+// that the chunks before it are never encoded and the first encoded chunk's
+// look-back never sees its predecessor published: the self-test of the
+// bounded wait (prism_lossless_wait_selftest).
+static int launch_encode_lookback(prism_handle* h, const uint8_t* planes, const Geometry& g, uint8_t* stream,
+                                  cudaStream_t st, int first_ticket, long long spin_limit) {
+  Small* s = small(h);
+  CK(cudaMemsetAsync(h->marks.p, 0, (size_t)g.chunks * sizeof(unsigned long long), st));
   CK(cudaMemsetAsync(&s->ticket, 0, sizeof(unsigned long long), st));
   // little-endian: the low byte alone makes the 64-bit ticket counter equal to first_ticket
-  if (first_ticket > 0) CK(cudaMemsetAsync(&s->ticket, first_ticket, 1, st));
+  CK(cudaMemsetAsync(&s->ticket, first_ticket, 1, st));
   CK(cudaMemsetAsync(&s->error_flag, 0, sizeof(int), st));
   size_t smem = sizeof(EncodeShared);
   CK(smem_limit<zbpc_encode_kernel>((int)smem));
   int blocks = (int)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * 4);
   prof_begin(h, kStEncode, st);
-  zbpc_encode_kernel<<<blocks, kZThreads, smem, st>>>(planes, g, stream, h->status.as<unsigned long long>(),
+  zbpc_encode_kernel<<<blocks, kZThreads, smem, st>>>(planes, g, stream, h->marks.as<unsigned long long>(),
                                                       &s->ticket, s->csbp, &s->lossless_size, &s->error_flag,
                                                       spin_limit);
   zbpc_finish_kernel<<<1, 32, 0, st>>>(stream, g, &s->lossless_size, &s->padded_size);
@@ -577,22 +609,11 @@ static int launch_decode(prism_handle* h, const uint8_t* stream, uint64_t stream
   return PRISM_OK;
 }
 
-// trailer (compress_merge, compressor.cu:139-151): use_md[4], reverse[4],
-// double range, size_t comp_size_bp[4][32], anchors
 template <class T>
 __global__ void trailer_kernel(uint8_t* stream, const uint64_t* padded, const PredParams<T>* p, const double* range,
                                const uint64_t* csbp, const T* anchors, uint64_t nanchors) {
-  uint8_t* tr = stream + *padded;
-  uint64_t total = 1040 + nanchors * sizeof(T);
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    uint8_t v;
-    if (i < 4) v = p->use_md[i];
-    else if (i < 8) v = p->reverse[i - 4];
-    else if (i < 16) v = reinterpret_cast<const uint8_t*>(range)[i - 8];
-    else if (i < 1040) v = reinterpret_cast<const uint8_t*>(csbp)[i - 16];
-    else v = reinterpret_cast<const uint8_t*>(anchors)[i - 1040];
-    tr[i] = v;
-  }
+  write_trailer(stream + *padded, p, range, csbp, anchors, nanchors,
+                (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x, ~0ull);
 }
 
 // the results of a pipeline call, stored into the handle's mapped host block
@@ -646,9 +667,10 @@ static int compress_t(prism_handle* h, const T* in, const Geometry& g, int mode,
   rc = launch_predict<T>(h, in, g, params_ptr<T>(h), h->anchors.as<T>(), h->qc.as<int32_t>(), st);
   if (rc) return rc;
   prof_end(h, kStPredict, st);
-  rc = launch_bitshuffle(h, h->qc.as<int32_t>(), g, nb, h->planes.as<uint8_t>(), st);
+  rc = launch_bitshuffle(h, h->qc.as<int32_t>(), g, nb, h->planes.as<uint8_t>(),
+                        h->marks.as<uint32_t>(), st);
   if (rc) return rc;
-  rc = launch_encode(h, h->planes.as<uint8_t>(), g, out, st);
+  rc = launch_encode(h, h->planes.as<uint8_t>(), h->planes.as<uint8_t>(), h->marks.as<uint32_t>(), g, out, st);
   if (rc) return rc;
   prof_begin(h, kStTrailer, st);
   trailer_kernel<T><<<64, 256, 0, st>>>(out, &s->padded_size, params_ptr<T>(h), &s->range, s->csbp,
@@ -714,7 +736,7 @@ int prism_create(prism_handle** out) {
 
 void prism_destroy(prism_handle* h) {
   if (!h) return;
-  DevBuf* bufs[] = {&h->qc, &h->planes, &h->status, &h->offs, &h->part, &h->wins, &h->ranges,
+  DevBuf* bufs[] = {&h->qc, &h->planes, &h->marks, &h->offs, &h->part, &h->wins, &h->ranges,
                     &h->anchors, &h->small, &h->dev_in, &h->dev_out, &h->zero_anchors, &h->prog_slots,
                     &h->sbatch, &h->qc_odd, &h->ext};
   for (DevBuf* b : bufs) b->release();
@@ -1275,7 +1297,7 @@ int prism_bitshuffle(prism_handle* h, const int32_t* d_codes, uint32_t nx, uint3
   int rc = ensure_common(h, g);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_bitshuffle(h, d_codes, g, progressive ? 1 : 0, d_planes, st);
+  rc = launch_bitshuffle(h, d_codes, g, progressive ? 1 : 0, d_planes, nullptr, st);
   if (rc) return rc;
   CK(cudaStreamSynchronize(st));
   return PRISM_OK;
@@ -1321,7 +1343,7 @@ int prism_lossless_encode(prism_handle* h, const uint8_t* d_planes, uint32_t nx,
   int rc = ensure_common(h, g);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_encode(h, d_planes, g, d_stream, st);
+  rc = launch_encode(h, d_planes, h->planes.as<uint8_t>(), nullptr, g, d_stream, st);
   if (rc) return rc;
   if (comp_size_bp) CK(cudaMemcpyAsync(comp_size_bp, small(h)->csbp, 1024, cudaMemcpyDeviceToHost, st));
   rc = finish(h, st);
@@ -1340,7 +1362,7 @@ int prism_lossless_wait_selftest(prism_handle* h, const uint8_t* d_planes, uint3
   int rc = ensure_common(h, g);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = launch_encode(h, d_planes, g, d_stream, st, 1, spin_limit);
+  rc = launch_encode_lookback(h, d_planes, g, d_stream, st, 1, spin_limit);
   if (rc) return rc;
   return finish(h, st);
 }

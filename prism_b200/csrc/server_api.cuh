@@ -90,7 +90,7 @@ constexpr int kPlanBatch = 32;
 uint64_t srv_workspace_bytes(uint32_t nx, uint32_t ny, uint32_t nz, int tsize) {
   Geometry g;
   make_geometry(nx, ny, nz, tsize, &g);
-  uint64_t b = qc_len(g) * 4 + g.aligned_size + 64 + (uint64_t)g.chunks * (8 + 2 * kChunkTableBytes) + g.anchors * 16 + 65536;
+  uint64_t b = qc_len(g) * 4 + g.aligned_size + 64 + marks_bytes(g) + (uint64_t)g.chunks * 2 * kChunkTableBytes + g.anchors * 16 + 65536;
   return b + b / 8;
 }
 

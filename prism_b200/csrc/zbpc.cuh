@@ -12,14 +12,13 @@
 // a byte is kept iff it differs from its predecessor, byte -1 being 0).
 // An all-zero chunk is just its 2-byte osize.
 //
-// B200 mapping.  Encode: persistent CTAs take chunk tickets from an atomic
-// counter (so every chunk's predecessors are already running), build the
-// payload in shared memory with block-wide prefix sums, and find their output
-// offset with a decoupled look-back over a per-chunk status word (bounded
-// spin: a stuck predecessor sets an error flag instead of hanging).  Decode:
-// offsets come from a scan of the size table; one CTA per chunk rebuilds the
-// bitmaps from the tail and scatters the bytes (a fill-forward is an inclusive
-// popcount prefix).
+// B200 mapping.  Encode: chunks are coded independently into a plane-sized
+// buffer, their offsets scanned, the payloads gathered (below); an entry point
+// without scratch has a one-launch form with tickets and a decoupled look-back
+// over a per-chunk status word (bounded spin: a stuck predecessor sets an
+// error flag instead of hanging).  Decode: offsets come from a scan of the
+// size table; one CTA per coded chunk rebuilds the bitmaps from the tail and
+// expands the bytes (a fill-forward is an inclusive popcount prefix).
 #pragma once
 #include "geometry.h"
 
@@ -56,6 +55,71 @@ __host__ __device__ __forceinline__ ChunkLoc locate_chunk(const Geometry& g, int
   int64_t rem = g.hastride[l] - c.offset * kChunk;
   c.osize = (int)(rem < kChunk ? rem : kChunk);
   c.last_of_plane = c.offset == cpp - 1;
+  return c;
+}
+
+// Chunk holding byte `off` of the plane buffer (host placement: level 3's 32
+// planes first, each plane cut into 16 KiB chunks; chunk ids follow the
+// bytes).  Offsets past the buffer map past the last chunk.
+__host__ __device__ __forceinline__ int64_t chunk_of_byte(const Geometry& g, int64_t off) {
+  int64_t hb = 0, cb = 0;
+  for (int l = 3; l >= 0; --l) {
+    const int64_t span = g.hastride[l] << 5;
+    if (off < hb + span || l == 0) {
+      const int64_t rel = off - hb, p = rel / g.hastride[l];
+      return cb + p * (g.chunks_level[l] >> 5) + (rel - p * g.hastride[l]) / kChunk;
+    }
+    hb += span;
+    cb += g.chunks_level[l];
+  }
+  return 0;
+}
+
+// Host placement of a byte of the plane buffer: its chunk, the chunk's level,
+// plane and byte range.  The byte is given with the level and plane whose
+// device placement it was computed from; the two placements drift apart by a
+// few bytes per plane, so the chunk is that plane's or a near one's and the
+// walk below takes a step or none (no division).
+struct HostChunk {
+  int64_t id, begin, end;
+  int level, plane;
+};
+__host__ __device__ __forceinline__ int64_t host_stride(const Geometry& g, int l) {
+  return l == 0 ? g.hastride[0] : (l == 1 ? g.hastride[1] : (l == 2 ? g.hastride[2] : g.hastride[3]));
+}
+__host__ __device__ __forceinline__ HostChunk chunk_near(const Geometry& g, int level, int plane, int64_t off) {
+  const int64_t h3 = g.hastride[3] << 5, h2 = h3 + (g.hastride[2] << 5), h1 = h2 + (g.hastride[1] << 5);
+  int l = level, p = plane;
+  int64_t stride = host_stride(g, l);
+  int64_t base = (l == 3 ? 0 : (l == 2 ? h3 : (l == 1 ? h2 : h1))) + p * stride;
+  while (off < base) {
+    if (p == 0) {
+      p = 31;
+      stride = host_stride(g, ++l);
+    } else {
+      --p;
+    }
+    base -= stride;
+  }
+  while (off >= base + stride && !(l == 0 && p == 31)) {
+    base += stride;
+    if (p == 31) {
+      p = 0;
+      stride = host_stride(g, --l);
+    } else {
+      ++p;
+    }
+  }
+  const int64_t k = (off - base) >> 14;
+  static_assert(kChunk == 1 << 14, "chunk index by shift");
+  HostChunk c;
+  c.level = l;
+  c.plane = p;
+  c.begin = base + k * kChunk;
+  c.end = c.begin + kChunk < base + stride ? c.begin + kChunk : base + stride;
+  const int64_t c3 = g.chunks_level[3], c2 = c3 + g.chunks_level[2], c1 = c2 + g.chunks_level[1];
+  const int64_t per = (l == 0 ? g.chunks_level[0] : (l == 1 ? g.chunks_level[1] : (l == 2 ? g.chunks_level[2] : c3))) >> 5;
+  c.id = (l == 3 ? 0 : (l == 2 ? c3 : (l == 1 ? c2 : c1))) + p * per + k;
   return c;
 }
 
@@ -335,8 +399,9 @@ __device__ __forceinline__ void encode_chunk(EncodeShared& sh, const uint8_t* __
   }
 }
 
-// Persistent encoder: one CTA (512 threads, 32 bytes each) per 16 KiB chunk,
-// four CTAs per SM, chunks handed out in order by a ticket counter.
+// One-launch encoder (prism_lossless_encode_static): one CTA (512 threads, 32
+// bytes each) per 16 KiB chunk, four CTAs per SM, chunks handed out in order by
+// a ticket counter.
 __global__ void __launch_bounds__(kZThreads, 4)
 zbpc_encode_kernel(const uint8_t* __restrict__ planes, Geometry g, uint8_t* __restrict__ stream,
                    unsigned long long* __restrict__ status, unsigned long long* __restrict__ ticket,
@@ -398,16 +463,17 @@ constexpr uint64_t kCodedMask = (1ull << 48) - 1;
 constexpr uint32_t kZeroChunkBytes = 2;
 constexpr int kScanThreads = 1024, kScanPer = 4, kScanItems = kScanThreads * kScanPer;
 
-// One launch for the whole table: a CTA scans kScanItems sizes and gets the
-// sums before them by reading the earlier part of the table itself (16 bits a
-// chunk: 0.5 MB for a 4.3 GB field, from L2), which costs less than a second
-// launch or a wait on the CTAs before it.
-__global__ void __launch_bounds__(kScanThreads)
-scan_chunks_kernel(const uint16_t* __restrict__ sizes, Geometry g, ChunkTable t) {
+// One launch for the whole table: a CTA (`cta` of the field's) scans
+// kScanItems sizes and gets the sums before them by reading the earlier part
+// of the table itself (16 bits a chunk: 0.5 MB for a 4.3 GB field, from L2),
+// which costs less than a second launch or a wait on the CTAs before it.
+// each(i, size, off, rank, coded) sees every chunk of the CTA.
+template <class F>
+__device__ __forceinline__ void scan_chunks(const uint16_t* __restrict__ sizes, const int64_t n, const int cta, F each) {
   __shared__ unsigned long long warp_tot[32], prior_b[32];
   __shared__ unsigned prior_c[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t n = g.chunks, base = (int64_t)blockIdx.x * kScanItems;
+  const int64_t base = (int64_t)cta * kScanItems;
   const bool vec = (reinterpret_cast<uintptr_t>(sizes) & 7) == 0;  // four sizes a load
   auto four = [&](int64_t i, uint32_t (&v)[4]) {
     if (vec && i + 4 <= n) {
@@ -469,16 +535,398 @@ scan_chunks_kernel(const uint16_t* __restrict__ sizes, Geometry g, ChunkTable t)
   for (int k = 0; k < kScanPer; ++k) {
     const int64_t i = i0 + k;
     if (i < n) {
-      t.offs[i] = (int64_t)off;
-      t.rank[i] = rank;
-      if (v[k] != kZeroChunkBytes) {
-        const ChunkLoc loc = locate_chunk(g, i);
-        t.coded[rank++] = pack_coded(off, v[k], (uint64_t)loc.base, (uint32_t)loc.osize);
-      }
+      const bool coded = v[k] != kZeroChunkBytes;
+      each(i, v[k], off, rank, coded);
+      rank += coded;
       off += v[k];
-      if (i == n - 1) t.rank[n] = rank;
     }
   }
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+scan_chunks_kernel(const uint16_t* __restrict__ sizes, Geometry g, ChunkTable t) {
+  scan_chunks(sizes, g.chunks, blockIdx.x, [&](int64_t i, uint32_t size, uint64_t off, uint32_t rank, bool coded) {
+    t.offs[i] = (int64_t)off;
+    t.rank[i] = rank;
+    if (coded) {
+      const ChunkLoc loc = locate_chunk(g, i);
+      t.coded[rank] = pack_coded(off, size, (uint64_t)loc.base, (uint32_t)loc.osize);
+    }
+    if (i == g.chunks - 1) t.rank[g.chunks] = rank + coded;
+  });
+}
+
+// ---------------- encode without look-back ----------------
+// The pipelines encode in three launches that wait for nothing on the device:
+//   encode_chunks   every chunk's size into the stream's size table and its
+//                   payload into the chunk's own place in a plane-sized buffer
+//                   (a coded payload is smaller than its chunk; a raw chunk
+//                   and an all-zero one need none).  The pipelines own their
+//                   plane buffer and encode it in place.
+//   scan            the payload offsets (scan_chunks) and the stream's totals
+//   gather          the payloads to their offsets in the stream
+// Against the one-launch encoder above (tickets, look-back) this moves the
+// container twice more through L2, but a chunk costs one barrier when it
+// turns out raw and two when it is coded, no CTA waits for its predecessors,
+// and chunks that the bit-plane shuffle knows to be zero are never read.  The
+// one-launch encoder stays for the entry point that has no scratch to put
+// payloads in.
+constexpr int kEncThreads = 256, kEncWarps = kEncThreads / 32, kEncCtas = 5;
+
+struct EncodeJob {
+  const uint8_t* planes;
+  uint8_t* slots;   // plane-sized, may be `planes`
+  uint16_t* sizes;  // the stream's size table
+};
+
+struct EncodeShared2 {
+  // payload staging: nonzero bytes (< osize) plus up to 2048 + 256 + 32 + 6
+  // bitmap bytes before the size check can reject the encoding
+  uint4 out[(kChunk + 2048 + 512) / 16];
+  uint32_t compact[16];
+  uint8_t bm1[256];
+  uint32_t scratch[2][kEncWarps];
+  int csz;
+};
+
+// bit j = byte j of w is nonzero
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {
+  const uint32_t t = (((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) | w) & 0x80808080u;  // bits 7, 15, 23, 31
+  return (t * 0x00204081u) >> 28;
+}
+
+// nibble of flags -> byte-permute selector that moves the flagged bytes
+// down, and 8 x their count
+__device__ __forceinline__ uint32_t compact_entry(int nibble) {
+  uint32_t sel = 0, kept = 0;
+  for (int j = 0; j < 4; ++j)
+    if ((nibble >> j) & 1) sel |= (uint32_t)j << (4 * kept++);
+  for (uint32_t k = kept; k < 4; ++k) sel |= 4u << (4 * k);
+  return sel | (8 * kept) << 16;
+}
+
+// The bytes of w (32, flagged by `bits`) that are kept, to out[pos ..]: few
+// are stored one by one (read again through L1), otherwise whole words are
+// assembled, the words shared with the neighbouring ranges byte by byte.
+__device__ __forceinline__ void compact_word(EncodeShared2& sh, const uint32_t (&w)[8], const uint8_t* src, uint32_t bits,
+                                             int pos, int most) {
+  uint8_t* out = reinterpret_cast<uint8_t*>(sh.out);
+  if (most <= 4) {
+    for (uint32_t b = bits; b; b &= b - 1) out[pos++] = src[__ffs(b) - 1];
+    return;
+  }
+  uint32_t* o32 = reinterpret_cast<uint32_t*>(sh.out);
+  int at = pos >> 2, head = pos & 3, fill = 8 * head;
+  uint32_t lo = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const uint32_t e = sh.compact[(bits >> (4 * q)) & 15u];
+    const uint32_t x = __byte_perm(w[q], 0u, e);
+    const uint32_t next = fill ? x >> (32 - fill) : 0u;  // what does not fit the open word
+    lo |= x << fill;
+    fill += e >> 16;
+    if (fill >= 32) {
+      if (head) {
+        for (int j = head; j < 4; ++j) out[4 * at + j] = (uint8_t)(lo >> (8 * j));
+        head = 0;
+      } else {
+        o32[at] = lo;
+      }
+      ++at;
+      fill -= 32;
+      lo = next;
+    }
+  }
+  for (int j = head; 8 * j < fill; ++j) out[4 * at + j] = (uint8_t)(lo >> (8 * j));
+}
+
+// Encode the chunk of `osize` bytes at `base` of the planes; returns its size
+// (uniform).  parity alternates between a CTA's chunks.
+__device__ __forceinline__ int encode_chunk_slot(EncodeShared2& sh, const uint8_t* planes, uint8_t* slots,
+                                                 const int64_t base, const int osize, const int parity) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint8_t* src = planes + base;
+  // words `first` and first + 32 of the 512-word zero-elimination bitmap, 32
+  // bytes each
+  const int first = 64 * warp + lane;
+  uint32_t wa[8], wb[8];
+  auto load = [&](uint32_t (&w)[8], int b0) {
+    const uint2* p = reinterpret_cast<const uint2*>(src + b0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint2 x = make_uint2(0, 0);
+      if (b0 + 8 * q < osize) x = p[q];
+      w[2 * q] = x.x;
+      w[2 * q + 1] = x.y;
+    }
+  };
+  load(wa, 32 * first);
+  load(wb, 32 * first + 1024);
+  uint32_t before = 0;  // the bitmap byte before the warp's first
+  if (lane == 0 && warp > 0 && 2048 * warp - 8 < osize) {
+    const uint2 x = *reinterpret_cast<const uint2*>(src + 2048 * warp - 8);
+    before = nonzero_bytes(x.x) | nonzero_bytes(x.y) << 4;
+  }
+  uint32_t ba = 0, bb = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    ba |= nonzero_bytes(wa[q]) << (4 * q);
+    bb |= nonzero_bytes(wb[q]) << (4 * q);
+  }
+  // flags of the bitmap bytes that differ from their predecessors
+  uint32_t prev_a = __shfl_up_sync(0xffffffffu, ba, 1) >> 24, prev_b = __shfl_up_sync(0xffffffffu, bb, 1) >> 24;
+  const uint32_t last_a = __shfl_sync(0xffffffffu, ba, 31) >> 24;
+  if (lane == 0) {
+    prev_a = before;
+    prev_b = last_a;
+  }
+  const uint32_t fa = nonzero_bytes(ba ^ (ba << 8 | prev_a)), fb = nonzero_bytes(bb ^ (bb << 8 | prev_b));
+  const uint32_t cnt = __popc(ba) | __popc(bb) << 16, fcnt = __popc(fa) | __popc(fb) << 16;
+  uint32_t incl = cnt, fincl = fcnt;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d), u = __shfl_up_sync(0xffffffffu, fincl, d);
+    if (lane >= d) {
+      incl += t;
+      fincl += u;
+    }
+  }
+  const uint32_t all = __shfl_sync(0xffffffffu, incl, 31), fall = __shfl_sync(0xffffffffu, fincl, 31);
+  // (kept bitmap bytes << 16 | nonzero bytes) of the warp; the chunk's sums
+  // are at most 2048 and 16384
+  uint32_t* scratch = sh.scratch[parity];
+  if (lane == 0) scratch[warp] = (all & 0xffffu) + (all >> 16) + (((fall & 0xffffu) + (fall >> 16)) << 16);
+  __syncthreads();
+  const uint32_t t = lane < kEncWarps ? scratch[lane] : 0u;
+  const uint32_t total = __reduce_add_sync(0xffffffffu, t);
+  const int nz = (int)(total & 0xffffu), c1 = (int)(total >> 16);
+  if (nz == 0) return (int)kZeroChunkBytes;
+  if (nz + c1 + 6 >= osize) return osize;
+  const uint32_t pre = __reduce_add_sync(0xffffffffu, lane < warp ? t : 0u);
+  // nonzero bytes, in order
+  uint8_t* out = reinterpret_cast<uint8_t*>(sh.out);
+  const uint32_t excl = incl - cnt;
+  compact_word(sh, wa, src + 32 * first, ba, (int)(pre & 0xffffu) + (int)(excl & 0xffffu),
+               (int)__reduce_max_sync(0xffffffffu, (unsigned)__popc(ba)));
+  compact_word(sh, wb, src + 32 * first + 1024, bb,
+               (int)(pre & 0xffffu) + (int)(all & 0xffffu) + (int)(excl >> 16),
+               (int)__reduce_max_sync(0xffffffffu, (unsigned)__popc(bb)));
+  // RE 2048 -> 256: the flagged bitmap bytes
+  {
+    const uint32_t fexcl = fincl - fcnt;
+    int r = nz + (int)(pre >> 16) + (int)(fexcl & 0xffffu);
+    for (uint32_t f = fa; f; f &= f - 1) out[r++] = (uint8_t)(ba >> (8 * (__ffs(f) - 1)));
+    r = nz + (int)(pre >> 16) + (int)(fall & 0xffffu) + (int)(fexcl >> 16);
+    for (uint32_t f = fb; f; f &= f - 1) out[r++] = (uint8_t)(bb >> (8 * (__ffs(f) - 1)));
+    const uint32_t oa = __shfl_down_sync(0xffffffffu, fa, 1), ob = __shfl_down_sync(0xffffffffu, fb, 1);
+    if ((lane & 1) == 0) {
+      sh.bm1[first >> 1] = (uint8_t)(fa | oa << 4);
+      sh.bm1[(first >> 1) + 16] = (uint8_t)(fb | ob << 4);
+    }
+  }
+  __syncthreads();
+  // The first two parts of the payload leave while warp 0 builds the rest,
+  // unless the size check can still reject the encoding: the slot may be the
+  // chunk itself, which then stays as it is.
+  const int head = nz + c1;
+  const bool certain = head + 6 + 256 + 32 < osize;
+  const int lead = certain ? head & ~7 : 0;  // bytes the other warps copy
+  uint2* dst = reinterpret_cast<uint2*>(slots + base);
+  const uint2* o2 = reinterpret_cast<const uint2*>(sh.out);
+  int csize = 0;
+  if (warp == 0) {
+    // RE 256 -> 32: lane l flags bm1 bytes 8l..8l+7
+    const uint2 b8 = reinterpret_cast<const uint2*>(sh.bm1)[lane];
+    uint32_t last = __shfl_up_sync(0xffffffffu, b8.y, 1) >> 24;
+    if (lane == 0) last = 0;
+    const uint32_t f2 = nonzero_bytes(b8.x ^ (b8.x << 8 | last)) |
+                        nonzero_bytes(b8.y ^ (b8.y << 8 | b8.x >> 24)) << 4;
+    const int cnt2 = __popc(f2);
+    const int incl2 = warp_incl_scan(cnt2, lane);
+    const int c2 = __shfl_sync(0xffffffffu, incl2, 31);
+    int r = head + incl2 - cnt2;
+    for (uint32_t f = f2; f; f &= f - 1) {
+      const int k = __ffs(f) - 1;
+      out[r++] = (uint8_t)((k < 4 ? b8.x : b8.y) >> (8 * (k & 3)));
+    }
+    // RE 32 -> 4: lane l flags bm2 byte l (= f2)
+    uint32_t prev2 = __shfl_up_sync(0xffffffffu, f2, 1);
+    if (lane == 0) prev2 = 0;
+    const uint32_t bal = __ballot_sync(0xffffffffu, f2 != prev2);
+    int pos = head + c2;
+    if (f2 != prev2) out[pos + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)f2;
+    pos += __popc(bal);
+    csize = pos + 6;
+    if (csize < osize) {
+      if (lane < 4) out[pos + lane] = (uint8_t)(bal >> (8 * lane));
+      if (lane == 0) {
+        out[pos + 4] = (uint8_t)osize;
+        out[pos + 5] = (uint8_t)(osize >> 8);
+      }
+    }
+    __syncwarp();
+    if (certain)
+      for (int i = (lead >> 3) + lane; 8 * i < csize; i += 32) dst[i] = o2[i];
+    else if (lane == 0) sh.csz = csize;
+  } else {
+    for (int i = tid - 32; 8 * i < lead; i += kEncThreads - 32) dst[i] = o2[i];
+  }
+  if (!certain) {
+    __syncthreads();
+    csize = sh.csz;
+    if (csize >= osize) return osize;
+    for (int i = tid; 8 * i < csize; i += kEncThreads) dst[i] = o2[i];
+  }
+  return csize;  // of warp 0 where `certain`
+}
+
+// The chunks of a CTA: rounds of kEncThreads chunk ids (every gridDim.x-th
+// one), a thread each; the all-zero ones are done with, the others are listed
+// and encoded one after the other by the CTA.  find(item) gives the job,
+// geometry and chunk id of an item.
+struct EncodeItem {
+  EncodeJob job;
+  int64_t base;
+  uint32_t id;
+  int osize;
+};
+template <class F>
+__device__ __forceinline__ void encode_items(EncodeShared2& sh, EncodeItem (&list)[kEncThreads], const uint64_t items,
+                                             F find) {
+  __shared__ int listed;
+  const int tid = threadIdx.x;
+  if (tid < 16) sh.compact[tid] = compact_entry(tid);
+  int parity = 0;
+  for (uint64_t i0 = blockIdx.x; i0 < items; i0 += (uint64_t)gridDim.x * kEncThreads) {
+    if (tid == 0) listed = 0;
+    __syncthreads();  // also: the previous round's list is no longer read
+    const uint64_t i = i0 + (uint64_t)tid * gridDim.x;
+    if (i < items) {
+      EncodeItem it;
+      if (find(i, it)) list[atomicAdd(&listed, 1)] = it;
+      else it.job.sizes[it.id] = (uint16_t)kZeroChunkBytes;
+    }
+    __syncthreads();
+    const int n = listed;
+    for (int k = 0; k < n; ++k) {
+      const EncodeItem& it = list[k];
+      const int csize = encode_chunk_slot(sh, it.job.planes, it.job.slots, it.base, it.osize, parity);
+      if (tid == 0) it.job.sizes[it.id] = (uint16_t)csize;
+      parity ^= 1;
+    }
+    __syncthreads();
+  }
+}
+
+constexpr int encode_smem_bytes() { return (int)(sizeof(EncodeShared2) + kEncThreads * sizeof(EncodeItem)); }
+
+// Offsets and totals of an encoded stream: payload offset per chunk, the
+// cumulative plane sizes, the header, the zero padding.
+struct StreamTotals {
+  uint64_t* comp_size_bp;
+  uint64_t* lossless_size;
+  uint64_t* padded_size;
+  int* error_flag;
+};
+__device__ __forceinline__ void scan_stream(uint8_t* stream, const Geometry& g, int64_t* offs, const StreamTotals& t,
+                                            int cta) {
+  const int64_t n = g.chunks;
+  scan_chunks(reinterpret_cast<const uint16_t*>(stream + 8), n, cta,
+              [&](int64_t i, uint32_t size, uint64_t off, uint32_t, bool) {
+    offs[i] = (int64_t)off;
+    const ChunkLoc loc = locate_chunk(g, i);
+    if (loc.last_of_plane) t.comp_size_bp[(3 - loc.level) * 32 + loc.plane] = off + size;
+    if (i == n - 1) {
+      const uint64_t total = 8 + 2 * (uint64_t)n + off + size, pad = (8 - total % 8) % 8;
+      for (uint64_t k = 0; k < pad; ++k) stream[total + k] = 0;
+      for (int k = 0; k < 8; ++k) stream[k] = (uint8_t)((uint64_t)g.aligned_size >> (8 * k));
+      *t.lossless_size = off + size;
+      *t.padded_size = total + pad;
+      *t.error_flag = 0;
+    }
+  });
+}
+__global__ void __launch_bounds__(kScanThreads)
+scan_stream_kernel(uint8_t* stream, Geometry g, int64_t* offs, StreamTotals t) {
+  scan_stream(stream, g, offs, t, blockIdx.x);
+}
+
+// Copy n bytes from an 8-byte aligned address to an arbitrarily aligned one:
+// head bytes, then aligned 32-bit words (each from two source words, loaded
+// once: the second is the next lane's), four in flight, then the tail.
+__device__ __forceinline__ void gather_copy(uint8_t* dst, const uint8_t* __restrict__ src, int n) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  int head = (int)((4 - ((uintptr_t)dst & 3)) & 3);
+  if (head > n) head = n;
+  const int words = (n - head) >> 2, have = (n + 3) >> 2;  // whole words out, source words
+  if (tid < head) dst[tid] = src[tid];
+  uint32_t* dw = reinterpret_cast<uint32_t*>(dst + head);
+  const uint32_t* sw = reinterpret_cast<const uint32_t*>(src);
+#pragma unroll 1
+  for (int w0 = tid; w0 - lane < words; w0 += 4 * kEncThreads) {  // warp-uniform trips
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int w = w0 + k * kEncThreads;
+      lo[k] = w < have ? __ldg(sw + w) : 0u;
+      hi[k] = (lane == 31 && w + 1 < have) ? __ldg(sw + w + 1) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int w = w0 + k * kEncThreads;
+      const uint32_t next = __shfl_down_sync(0xffffffffu, lo[k], 1);
+      if (lane != 31) hi[k] = next;
+      if (w < words) dw[w] = __funnelshift_r(lo[k], hi[k], 8 * head);
+    }
+  }
+  const int done = head + 4 * words;
+  if (tid < n - done) dst[done + tid] = src[done + tid];
+}
+
+// Payloads to their places in the stream, in rounds as encode_items.
+struct GatherItem {
+  const uint8_t* src;
+  uint8_t* dst;
+  int n;
+};
+template <class F>
+__device__ __forceinline__ void gather_items(GatherItem (&list)[kEncThreads], const uint64_t items, F find) {
+  __shared__ int listed;
+  const int tid = threadIdx.x;
+  for (uint64_t i0 = blockIdx.x; i0 < items; i0 += (uint64_t)gridDim.x * kEncThreads) {
+    if (tid == 0) listed = 0;
+    __syncthreads();
+    const uint64_t i = i0 + (uint64_t)tid * gridDim.x;
+    if (i < items) {
+      GatherItem it;
+      if (find(i, it)) list[atomicAdd(&listed, 1)] = it;
+    }
+    __syncthreads();
+    const int n = listed;
+    for (int k = 0; k < n; ++k) gather_copy(list[k].dst, list[k].src, list[k].n);
+    __syncthreads();
+  }
+}
+// Item of chunk `id`; an all-zero chunk's two bytes are written here.
+__device__ __forceinline__ bool gather_chunk(const EncodeJob& job, const Geometry& g, uint8_t* stream,
+                                             const int64_t* offs, int64_t id, GatherItem& it) {
+  const ChunkLoc loc = locate_chunk(g, id);
+  it.n = job.sizes[id];
+  it.dst = stream + 8 + 2 * g.chunks + offs[id];
+  if (it.n == (int)kZeroChunkBytes) {
+    it.dst[0] = (uint8_t)loc.osize;
+    it.dst[1] = (uint8_t)(loc.osize >> 8);
+    return false;
+  }
+  it.src = (it.n == loc.osize ? job.planes : job.slots) + loc.base;
+  return true;
+}
+__global__ void __launch_bounds__(kEncThreads)
+gather_stream_kernel(const EncodeJob job, Geometry g, uint8_t* stream, const int64_t* __restrict__ offs) {
+  __shared__ GatherItem list[kEncThreads];
+  gather_items(list, (uint64_t)g.chunks, [&](uint64_t i, GatherItem& it) {
+    return gather_chunk(job, g, stream, offs, (int64_t)i, it);
+  });
 }
 
 constexpr int kDecThreads = 256, kDecWarps = kDecThreads / 32;
@@ -586,71 +1034,6 @@ __device__ __forceinline__ void expand_word(const DecodeShared& sh, uint4* stage
   }
   p0 = make_uint4(w[0], w[1], w[2], w[3]);
   p1 = make_uint4(w[4], w[5], w[6], w[7]);
-}
-
-// Chunk holding byte `off` of the plane buffer (host placement: level 3's 32
-// planes first, each plane cut into 16 KiB chunks; chunk ids follow the
-// bytes).  Offsets past the buffer map past the last chunk.
-__host__ __device__ __forceinline__ int64_t chunk_of_byte(const Geometry& g, int64_t off) {
-  int64_t hb = 0, cb = 0;
-  for (int l = 3; l >= 0; --l) {
-    const int64_t span = g.hastride[l] << 5;
-    if (off < hb + span || l == 0) {
-      const int64_t rel = off - hb, p = rel / g.hastride[l];
-      return cb + p * (g.chunks_level[l] >> 5) + (rel - p * g.hastride[l]) / kChunk;
-    }
-    hb += span;
-    cb += g.chunks_level[l];
-  }
-  return 0;
-}
-
-// Host placement of a byte of the plane buffer: its chunk, the chunk's level,
-// plane and byte range.  The byte is given with the level and plane whose
-// device placement it was computed from; the two placements drift apart by a
-// few bytes per plane, so the chunk is that plane's or a near one's and the
-// walk below takes a step or none (no division).
-struct HostChunk {
-  int64_t id, begin, end;
-  int level, plane;
-};
-__host__ __device__ __forceinline__ int64_t host_stride(const Geometry& g, int l) {
-  return l == 0 ? g.hastride[0] : (l == 1 ? g.hastride[1] : (l == 2 ? g.hastride[2] : g.hastride[3]));
-}
-__host__ __device__ __forceinline__ HostChunk chunk_near(const Geometry& g, int level, int plane, int64_t off) {
-  const int64_t h3 = g.hastride[3] << 5, h2 = h3 + (g.hastride[2] << 5), h1 = h2 + (g.hastride[1] << 5);
-  int l = level, p = plane;
-  int64_t stride = host_stride(g, l);
-  int64_t base = (l == 3 ? 0 : (l == 2 ? h3 : (l == 1 ? h2 : h1))) + p * stride;
-  while (off < base) {
-    if (p == 0) {
-      p = 31;
-      stride = host_stride(g, ++l);
-    } else {
-      --p;
-    }
-    base -= stride;
-  }
-  while (off >= base + stride && !(l == 0 && p == 31)) {
-    base += stride;
-    if (p == 31) {
-      p = 0;
-      stride = host_stride(g, --l);
-    } else {
-      ++p;
-    }
-  }
-  const int64_t k = (off - base) >> 14;
-  static_assert(kChunk == 1 << 14, "chunk index by shift");
-  HostChunk c;
-  c.level = l;
-  c.plane = p;
-  c.begin = base + k * kChunk;
-  c.end = c.begin + kChunk < base + stride ? c.begin + kChunk : base + stride;
-  const int64_t c3 = g.chunks_level[3], c2 = c3 + g.chunks_level[2], c1 = c2 + g.chunks_level[1];
-  const int64_t per = (l == 0 ? g.chunks_level[0] : (l == 1 ? g.chunks_level[1] : (l == 2 ? g.chunks_level[2] : c3))) >> 5;
-  c.id = (l == 3 ? 0 : (l == 2 ? c3 : (l == 1 ? c2 : c1))) + p * per + k;
-  return c;
 }
 
 // Which chunks a decode leaves as zeros: the all-zero ones and, when

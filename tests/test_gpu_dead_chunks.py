@@ -1,4 +1,6 @@
-"""Decoding that skips all-zero and unselected chunks.
+"""Encoding and decoding that skip all-zero (and unselected) chunks.
+
+The encoder does not read chunks whose shuffle items had no nonzero byte.
 
 The decoder leaves such chunks of the plane buffer alone but for their ends,
 and the inverse shuffle skips the rows that lie in them.  The host chunk
@@ -38,13 +40,15 @@ def env():
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("dims", SHAPES)
-def test_decompress_matches_oracle(env, dims, dtype):
+def test_round_trip_matches_oracle(env, dims, dtype):
     torch, P, h = env
     data = field(dims, dtype, sum(dims))
     for bound in (1e-6, 1e-3):  # the tight one first: it fills the plane buffer
         ctx = P.Context(*dims, np.dtype(dtype), P.REL, bound, False)
         comp = P.Compressor(ctx, h)
         cont = comp.compress_pipeline(torch.from_numpy(data).cuda()).clone()
+        want, _, _ = O.compress(data, ctx.error_mode, bound, 1, force=O.intp(*comp.flags))
+        assert cont.cpu().numpy().tobytes() == want, bound
         got = comp.decompress_pipeline(cont).cpu().numpy()
         want = O.decompress(cont.cpu().numpy().tobytes(), ctx.shape, dtype, ctx.error_mode, bound)
         assert np.array_equal(got.view(np.uint8), want.view(np.uint8)), bound
