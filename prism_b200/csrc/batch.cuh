@@ -14,6 +14,7 @@
 #pragma once
 #include "autotune.cuh"
 #include "bitplane.cuh"
+#include "flat.cuh"
 #include "predict.cuh"
 #include "zbpc.cuh"
 
@@ -255,6 +256,25 @@ batch_predict_persistent_kernel(const BatchField* __restrict__ fields, const int
     batch_tile_call<T, PART>(*reinterpret_cast<CompressSmem<T>*>(smem_raw), sg, &fields[gidx[e]],
                              (uint32_t)(item - prefix[e]));
   }
+}
+
+// The tiles of the group's fields with one plane, kFlatWarps a CTA (an item).
+template <class T>
+__global__ void __launch_bounds__(kFlatWarps * 32)
+batch_flat_kernel(const BatchField* __restrict__ fields, const int* __restrict__ gidx,
+                  const uint64_t* __restrict__ prefix, int n) {
+  __shared__ T win[kFlatWarps][kFlatWin];
+  __shared__ __align__(16) Geometry g;
+  const int e = find_field(prefix, n, blockIdx.x);
+  const BatchField& f = fields[gidx[e]];
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(&f.g);
+  for (int i = threadIdx.x; i < (int)(sizeof(Geometry) / 4); i += kFlatWarps * 32)
+    reinterpret_cast<uint32_t*>(&g)[i] = src[i];
+  __syncthreads();
+  const uint32_t tile = (uint32_t)(blockIdx.x - prefix[e]) * kFlatWarps + (threadIdx.x >> 5);
+  if (tile < g.ax * g.ay)
+    flat_compress_tile(win[threadIdx.x >> 5], reinterpret_cast<const T*>(f.in), g, tile,
+                       reinterpret_cast<const PredParams<T>*>(f.st->params), reinterpret_cast<T*>(f.anchors), f.qc);
 }
 
 // leftover_fill_kernel over the ranges of all fields

@@ -32,6 +32,8 @@ struct prism_batch {
     void* d_partial = nullptr;
     uint64_t* d_tile_prefix[2] = {nullptr, nullptr};
     uint64_t tiles[2] = {0, 0};
+    uint64_t* d_flat_prefix = nullptr;
+    uint64_t flat_items = 0;
     uint64_t* d_tr_prefix = nullptr;
     uint64_t tr_items = 0;
   } grp[2];  // [0] float, [1] double
@@ -116,6 +118,11 @@ template <class T>
 int enqueue_group_predict(prism_batch* b, const prism_batch::Group& gr, int g, int ctas, cudaStream_t st,
                           uint64_t& launches) {
   const int smem = compress_smem_bytes<T>();
+  if (gr.flat_items) {
+    batch_flat_kernel<T><<<(unsigned)gr.flat_items, kFlatWarps * 32, 0, st>>>(b->d_fields, gr.d_idx, gr.d_flat_prefix,
+                                                                              gr.n);
+    ++launches;
+  }
   // ctas > 0: persistent CTAs (ctas per SM) on the tile counter; 0: one CTA
   // per tile
   for (int part = 0; part < 2; ++part) {
@@ -299,7 +306,7 @@ int batch_plan(prism_batch* b) {
   std::vector<std::pair<size_t, uint64_t>> zero_rel;  // (field qc offset in ints, len) resolved later
   struct GroupHost {
     std::vector<int> idx;
-    std::vector<uint64_t> ext{0}, win{0}, tile0{0}, tile1{0}, tr{0};
+    std::vector<uint64_t> ext{0}, win{0}, tile0{0}, tile1{0}, flat{0}, tr{0};
     std::vector<BatchWindow> wins;
   } gh[2];
   Carve cv;
@@ -351,8 +358,10 @@ int batch_plan(prism_batch* b) {
     std::vector<SampleWindow> w = sample_grid(g.nx, g.ny, g.nz);
     for (const SampleWindow& sw : w) G.wins.push_back(BatchWindow{sw, i, 0});
     G.win.push_back(G.win.back() + w.size());
-    G.tile0.push_back(G.tile0.back() + tiles_in_part(g, 0));
-    G.tile1.push_back(G.tile1.back() + tiles_in_part(g, 1));
+    const bool flat = is_flat(g);
+    G.tile0.push_back(G.tile0.back() + (flat ? 0 : tiles_in_part(g, 0)));
+    G.tile1.push_back(G.tile1.back() + (flat ? 0 : tiles_in_part(g, 1)));
+    G.flat.push_back(G.flat.back() + (flat ? flat_ctas(g) : 0));
     const uint64_t tr_bytes = 1040 + g.anchors * (uint64_t)d.dtype_size;
     G.tr.push_back(G.tr.back() + (tr_bytes + kBatchTrailerSeg - 1) / kBatchTrailerSeg);
     (void)e;
@@ -367,7 +376,7 @@ int batch_plan(prism_batch* b) {
   size_t o_post = cv.take<BatchLastCta>(std::max<size_t>(post.size(), 1));
   size_t o_scan = cv.take<BatchLastCta>(std::max<size_t>(scan.size(), 1));
   size_t o_zero = cv.take<BatchZero>(std::max<size_t>(zero_rel.size(), 1));
-  struct GroupOff { size_t idx, ext, extpart, win, wins, partial, t0, t1, tr; } go[2];
+  struct GroupOff { size_t idx, ext, extpart, win, wins, partial, t0, t1, flat, tr; } go[2];
   for (int k = 0; k < 2; ++k) {
     GroupHost& G = gh[k];
     const int gn = (int)G.idx.size();
@@ -380,6 +389,7 @@ int batch_plan(prism_batch* b) {
     go[k].partial = cv.take<unsigned char>(15 * ts * std::max<size_t>(G.wins.size(), 1));
     go[k].t0 = cv.take<uint64_t>(gn + 1);
     go[k].t1 = cv.take<uint64_t>(gn + 1);
+    go[k].flat = cv.take<uint64_t>(gn + 1);
     go[k].tr = cv.take<uint64_t>(gn + 1);
   }
   cudaError_t e = cudaMalloc((void**)&b->dev, cv.off);
@@ -443,6 +453,8 @@ int batch_plan(prism_batch* b) {
     gr.d_tile_prefix[1] = reinterpret_cast<uint64_t*>(base + go[k].t1);
     gr.tiles[0] = G.tile0.back();
     gr.tiles[1] = G.tile1.back();
+    gr.d_flat_prefix = reinterpret_cast<uint64_t*>(base + go[k].flat);
+    gr.flat_items = G.flat.back();
     gr.d_tr_prefix = reinterpret_cast<uint64_t*>(base + go[k].tr);
     gr.tr_items = G.tr.back();
     if (!gr.n) continue;
@@ -452,6 +464,7 @@ int batch_plan(prism_batch* b) {
     BCK(up(gr.d_wins, G.wins.data(), sizeof(BatchWindow) * G.wins.size()));
     BCK(up(gr.d_tile_prefix[0], G.tile0.data(), sizeof(uint64_t) * (gr.n + 1)));
     BCK(up(gr.d_tile_prefix[1], G.tile1.data(), sizeof(uint64_t) * (gr.n + 1)));
+    BCK(up(gr.d_flat_prefix, G.flat.data(), sizeof(uint64_t) * (gr.n + 1)));
     BCK(up(gr.d_tr_prefix, G.tr.data(), sizeof(uint64_t) * (gr.n + 1)));
   }
   // ---- occupancy limits of the persistent kernels ----

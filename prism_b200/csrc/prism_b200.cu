@@ -19,6 +19,7 @@
 #include "../../include/prism_b200.h"
 #include "autotune.cuh"
 #include "bitplane.cuh"
+#include "flat.cuh"
 #include "geometry.h"
 #include "predict.cuh"
 #include "report.cuh"
@@ -302,10 +303,17 @@ static cudaError_t smem_limit(int bytes) {
 }
 
 // The tile kernels run as two launches: interior tiles (part 0) and the tiles
-// on the field's last slabs (part 1), on two streams.
+// on the field's last slabs (part 1), on two streams; fields with one plane
+// take the warp-per-tile kernels.
 template <class T>
 static int launch_predict(prism_handle* h, const T* in, const Geometry& g, const PredParams<T>* pp, T* anchors,
                           int32_t* qc, cudaStream_t st) {
+  if (is_flat(g)) {  // a 3-D tile would spend a CTA on 256 points (flat.cuh)
+    flat_compress_kernel<T><<<(unsigned)flat_ctas(g), kFlatWarps * 32, 0, st>>>(in, g, pp, anchors, qc);
+    h->launches += 1;
+    CK(cudaGetLastError());
+    return PRISM_OK;
+  }
   const int smem = compress_smem_bytes<T>();
   constexpr auto k0 = predict_compress_kernel<T, 0>;
   constexpr auto k1 = predict_compress_kernel<T, 1>;
@@ -322,6 +330,12 @@ static int launch_predict(prism_handle* h, const T* in, const Geometry& g, const
 template <class T, bool PROG>
 static int launch_reconstruct(prism_handle* h, const int32_t* qc, const T* anchors, const Geometry& g,
                               const PredParams<T>* pp, const T* old, T* out, cudaStream_t st) {
+  if (is_flat(g)) {
+    flat_reconstruct_kernel<T, PROG><<<(unsigned)flat_ctas(g), kFlatWarps * 32, 0, st>>>(qc, anchors, g, pp, old, out);
+    h->launches += 1;
+    CK(cudaGetLastError());
+    return PRISM_OK;
+  }
   const int smem0 = recon_smem_bytes<T>(), smem1 = recon_smem_bytes<T>();
   constexpr auto k0 = reconstruct_kernel<T, PROG, 0>;
   constexpr auto k1 = reconstruct_kernel<T, PROG, 1>;
