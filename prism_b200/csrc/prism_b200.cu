@@ -76,6 +76,7 @@ struct HostResult {
   int pad;
   unsigned char params[256];
   double errors[16];
+  StatPart stat;
 };
 
 }  // namespace
@@ -1651,12 +1652,11 @@ int prism_statistics(prism_handle* h, const void* d_original, const void* d_data
     stats_kernel<float><<<blocks, kStatThreads, 0, st>>>((const float*)d_original, (const float*)d_data, n, part);
   else
     stats_kernel<double><<<blocks, kStatThreads, 0, st>>>((const double*)d_original, (const double*)d_data, n, part);
-  stats_final_kernel<<<1, 32, 0, st>>>(part, blocks);
+  stats_final_kernel<<<1, kStatThreads, 0, st>>>(part, blocks, &h->host_dev->stat);
   h->launches += 2;
   CK(cudaGetLastError());
-  StatPart r;
-  CK(cudaMemcpyAsync(&r, part, sizeof(r), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  const StatPart r = h->host->stat;
   const double range = r.mx - r.mn, mse = r.l2 / (double)n;
   out[0] = r.maxe;
   out[1] = r.maxe / range;
