@@ -149,11 +149,19 @@ __device__ __forceinline__ void autotune_window(T* win, T* red, const T* __restr
 #pragma unroll
   for (int d = 0; d < 3; ++d) { t.gs[d] = w.gs[d]; t.notlast_[d] = w.gs[d] + 16u < t.dim[d]; }
   const uint64_t sy = g.nx, sz = (uint64_t)g.nx * g.ny;
-  for (int i = threadIdx.x; i < kWinVol; i += blockDim.x) {
-    int x = i % kWin, y = (i / kWin) % kWin, z = i / (kWin * kWin);
-    T v = T(0);
-    if (t.in_data(x, y, z)) v = data[(uint64_t)(t.gs[0] + x) + (uint64_t)(t.gs[1] + y) * sy + (uint64_t)(t.gs[2] + z) * sz];
-    win[i] = v;
+  constexpr int kBatch = 10, kFill = kBatch * kAttThreads;  // loads in flight, two batches
+  for (int i0 = 0; i0 < kWinVol; i0 += kFill) {
+    T v[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const int i = i0 + k * kAttThreads + threadIdx.x, x = i % kWin, y = (i / kWin) % kWin, z = i / (kWin * kWin);
+      v[k] = T(0);
+      if (i < kWinVol && t.in_data(x, y, z))
+        v[k] = __ldg(data + (uint64_t)(t.gs[0] + x) + (uint64_t)(t.gs[1] + y) * sy + (uint64_t)(t.gs[2] + z) * sz);
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k)
+      if (i0 + k * kAttThreads + threadIdx.x < kWinVol) win[i0 + k * kAttThreads + threadIdx.x] = v[k];
   }
   __syncthreads();
   if (biy == 0) {
@@ -179,14 +187,6 @@ __device__ __forceinline__ void autotune_window(T* win, T* red, const T* __restr
     T s = block_sum(e, red);
     if (threadIdx.x == 0) out[9 + biy] = s;
   }
-}
-
-template <class T>
-__global__ void __launch_bounds__(kAttThreads)
-autotune_kernel(const T* __restrict__ data, Geometry g, const SampleWindow* __restrict__ wins, T* __restrict__ partial) {
-  __shared__ T win[kWinVol];
-  __shared__ T red[kAttThreads];
-  autotune_window<T>(win, red, data, g, wins[blockIdx.x], blockIdx.y, partial + (size_t)blockIdx.x * 15);
 }
 
 // Field parameters, computed on the device so nothing waits for the host:
@@ -253,26 +253,13 @@ __device__ __forceinline__ void compute_params(int mode, double bound, const dou
   if (eb_out) *eb_out = eb;
 }
 
-// One warp: lane k < 15 sums variant k's errors over the windows in window
-// order (the same sums, in the same order, as a single thread would form),
-// then lane 0 decides.
+// Parameters with the flags of a container (or forced ones).
 template <class T>
 __global__ void params_kernel(int mode, double bound, const double* __restrict__ range, double alpha,
-                              const T* __restrict__ partial, int nwin, const uint8_t* __restrict__ flags_in,
-                              int maxlevel, PredParams<T>* __restrict__ out, T* __restrict__ errors_out,
+                              const uint8_t* __restrict__ flags_in, int maxlevel, PredParams<T>* __restrict__ out,
                               double* __restrict__ eb_out) {
-  __shared__ T sums[15];
-  if (blockIdx.x != 0) return;
-  const int k = threadIdx.x;
-  if (partial && k < 15) {
-    T s = T(0);
-    for (int w = 0; w < nwin; ++w) s = Fp<T>::add(s, partial[(size_t)w * 15 + k]);
-    sums[k] = s;
-  }
-  __syncthreads();
-  if (k != 0) return;
-  compute_params<T>(mode, bound, range, alpha, partial, nwin, flags_in, maxlevel, out, errors_out, eb_out,
-                    partial ? sums : nullptr);
+  if (threadIdx.x == 0 && blockIdx.x == 0)
+    compute_params<T>(mode, bound, range, alpha, nullptr, 0, flags_in, maxlevel, out, nullptr, eb_out);
 }
 
 // Global min / max (compressor.cu:230-302): per-block partials, then one block.
@@ -307,14 +294,13 @@ template <> struct Vec16<float> {
 // compares below (above) it, so a NaN is skipped unless it is in[0], and the
 // result does not depend on the order in which values are folded.
 template <class T>
-__global__ void __launch_bounds__(kExtThreads)
-extrema_kernel(const T* __restrict__ in, uint64_t n, T* __restrict__ part) {
+__device__ __forceinline__ void extrema_cta(const T* __restrict__ in, uint64_t n, T* __restrict__ part, int cta, int ncta,
+                                            T* smin, T* smax) {
   using V = typename Vec16<T>::type;
   constexpr uint64_t W = 16 / sizeof(T);
-  __shared__ T smin[kExtThreads], smax[kExtThreads];
   T mn = in[0], mx = in[0];
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t stride = (uint64_t)ncta * blockDim.x;
+  const uint64_t tid = (uint64_t)cta * blockDim.x + threadIdx.x;
   // values before the first 16-byte boundary, the 16-byte vectors (four
   // independent loads in flight), the values after the last whole vector
   uint64_t head = ((16 - (reinterpret_cast<uintptr_t>(in) & 15)) & 15) / sizeof(T);
@@ -351,7 +337,14 @@ extrema_kernel(const T* __restrict__ in, uint64_t n, T* __restrict__ part) {
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) { part[2 * blockIdx.x] = smin[0]; part[2 * blockIdx.x + 1] = smax[0]; }
+  if (threadIdx.x == 0) { part[2 * cta] = smin[0]; part[2 * cta + 1] = smax[0]; }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kExtThreads)
+extrema_kernel(const T* __restrict__ in, uint64_t n, T* __restrict__ part) {
+  __shared__ T smin[kExtThreads], smax[kExtThreads];
+  extrema_cta(in, n, part, blockIdx.x, gridDim.x, smin, smax);
 }
 
 // one warp folds the per-block extrema (min/max are order independent)
@@ -378,6 +371,90 @@ __global__ void extrema_final_kernel(const T* __restrict__ part, int nblocks, do
       minmax[1] = (double)mx;
     }
   }
+}
+
+// ---- the front of a compression in two launches -----------------------------
+// What a compression does before the predictor needs no more than the field:
+// the auto-tune windows (the longest, first in the grid), the extrema scan
+// (four CTAs of 256 threads an SM keep the copy bandwidth beside them) and the
+// code padding run as one launch over CTA ranges; the second folds the
+// extrema and window sums and computes the parameters.  Five launches, four
+// memsets and a second stream's events otherwise, 15-20 us of a small call.
+struct ZeroList {  // int32 ranges to zero (code_padding)
+  int32_t* p[4];
+  uint64_t n[4];
+};
+
+template <class T>
+__global__ void __launch_bounds__(kAttThreads)
+front_kernel(const T* __restrict__ in, Geometry g, const SampleWindow* __restrict__ wins, int natt, T* __restrict__ partial,
+             int next, T* __restrict__ ext, ZeroList zero) {
+  __shared__ T win[kWinVol];
+  __shared__ T red[2 * kAttThreads];
+  int b = blockIdx.x;
+  if (b < natt) {
+    autotune_window<T>(win, red, in, g, wins[b / 6], b % 6, partial + (size_t)(b / 6) * 15);
+    return;
+  }
+  b -= natt;
+  if (b < next) {
+    extrema_cta(in, g.n, ext, b, next, red, red + kAttThreads);
+    return;
+  }
+  b -= next;
+  int32_t* p = b == 0 ? zero.p[0] : (b == 1 ? zero.p[1] : (b == 2 ? zero.p[2] : zero.p[3]));
+  const uint64_t n = b == 0 ? zero.n[0] : (b == 1 ? zero.n[1] : (b == 2 ? zero.n[2] : zero.n[3]));
+  for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) p[i] = 0;
+}
+
+// One CTA: warp 0's lane k < 15 sums variant k's errors over the windows in
+// window order (the same sums, in the same order, as a single thread would
+// form), the other warps fold the extrema (order independent), thread 0
+// decides.  next = 0: the range is 1 (an absolute bound).
+template <class T>
+__global__ void __launch_bounds__(kAttThreads)
+front_params_kernel(int mode, double bound, const T* __restrict__ ext, int next, double alpha,
+                    const T* __restrict__ partial, int nwin, double* __restrict__ range, PredParams<T>* __restrict__ out,
+                    T* __restrict__ errors_out, double* __restrict__ eb_out) {
+  __shared__ T sums[15], mns[kAttThreads / 32], mxs[kAttThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp == 0) {
+    if (lane < 15) {
+      T s = T(0);
+      for (int w = 0; w < nwin; ++w) s = Fp<T>::add(s, partial[(size_t)w * 15 + lane]);
+      sums[lane] = s;
+    }
+  } else if (next > 0) {
+    T mn = ext[0], mx = ext[1];
+    for (int b = threadIdx.x - 32; b < next; b += kAttThreads - 32) {
+      const T a = ext[2 * b], c = ext[2 * b + 1];
+      mn = a < mn ? a : mn;
+      mx = c > mx ? c : mx;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      const T a = __shfl_xor_sync(0xffffffffu, mn, d), c = __shfl_xor_sync(0xffffffffu, mx, d);
+      mn = a < mn ? a : mn;
+      mx = c > mx ? c : mx;
+    }
+    if (lane == 0) {
+      mns[warp] = mn;
+      mxs[warp] = mx;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double r = 1.0;
+  if (next > 0) {
+    T mn = mns[1], mx = mxs[1];
+    for (int w = 2; w < kAttThreads / 32; ++w) {
+      mn = mns[w] < mn ? mns[w] : mn;
+      mx = mxs[w] > mx ? mxs[w] : mx;
+    }
+    r = __dsub_rn((double)mx, (double)mn);
+  }
+  *range = r;
+  compute_params<T>(mode, bound, &r, alpha, partial, nwin, nullptr, 4, out, errors_out, eb_out, sums);
 }
 
 }  // namespace prism_b200

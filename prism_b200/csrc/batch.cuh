@@ -160,7 +160,7 @@ __global__ void batch_extrema_final_kernel(const BatchField* __restrict__ fields
   if (lane == 0) f.st->range = __dsub_rn((double)mx, (double)mn);
 }
 
-// grid (windows of the group, 6): partial[window][15] as autotune_kernel
+// grid (windows of the group, 6): partial[window][15] as front_kernel
 template <class T>
 __global__ void __launch_bounds__(kAttThreads)
 batch_autotune_kernel(const BatchField* __restrict__ fields, const BatchWindow* __restrict__ wins,
@@ -342,7 +342,7 @@ batch_scan_kernel(const BatchField* __restrict__ fields, const BatchLastCta* __r
 __global__ void __launch_bounds__(kEncThreads)
 batch_gather_kernel(const BatchField* __restrict__ fields, const uint64_t* __restrict__ prefix, int n, uint64_t items) {
   __shared__ GatherItem list[kEncThreads];
-  gather_items(list, items, [&](uint64_t i, GatherItem& it) {
+  gather_items(list, items, blockIdx.x, gridDim.x, [&](uint64_t i, GatherItem& it) {
     const int e = find_field(prefix, n, i);
     const BatchField& f = fields[e];
     return gather_chunk(batch_job(f), f.g, f.out, f.offs, (int64_t)(i - prefix[e]), it);

@@ -1328,6 +1328,28 @@ predict_compress_kernel(const T* __restrict__ data, Geometry g, const PredParams
   compress_tile<T, PART == 1>(sm, data, g, bi, pp, anchors, qc);
 }
 
+// Both parts in one launch, the (longer) last-slab tiles first: for fields
+// whose tiles are all on the GPU at once, where a second stream's events cost
+// more than the wider register budget of the joined kernel: the two parts of
+// a 64x48x40 float field (12 and 16 us) took 19 us from the first start to the
+// last end and two gaps of 8 us around them.
+template <class T>
+__global__ void __launch_bounds__(kPredThreads, 4)
+predict_compress_both_kernel(const T* __restrict__ data, Geometry g, const PredParams<T>* __restrict__ pp,
+                             T* __restrict__ anchors, int32_t* __restrict__ qc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  CompressSmem<T>& sm = *reinterpret_cast<CompressSmem<T>*>(smem_raw);
+  const uint32_t edge = (uint32_t)tiles_in_part(g, 1);
+  uint32_t bi[3];
+  if (blockIdx.x < edge) {
+    tile_of_index<1>(g, blockIdx.x, bi);
+    compress_tile<T, true>(sm, data, g, bi, pp, anchors, qc);
+  } else {
+    tile_of_index<0>(g, blockIdx.x - edge, bi);
+    compress_tile<T, false>(sm, data, g, bi, pp, anchors, qc);
+  }
+}
+
 // Reconstruction: anchors + codes -> values (interpolation_reverse
 // :2177-2207); PROG adds the previous values (interpolation_progressive_reverse
 // :2209-2239, shmem2global_data_progressive :1123-1147).  All codes the tile

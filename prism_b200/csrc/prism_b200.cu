@@ -316,11 +316,19 @@ static int launch_predict(prism_handle* h, const T* in, const Geometry& g, const
     return PRISM_OK;
   }
   const int smem = compress_smem_bytes<T>();
+  const uint64_t n0 = tiles_in_part(g, 0), n1 = tiles_in_part(g, 1);
+  if (n0 > 0 && n0 + n1 <= (uint64_t)h->sm_count * 4) {  // one wave of the joined kernel
+    constexpr auto k = predict_compress_both_kernel<T>;
+    CK(smem_limit<k>(smem));
+    k<<<(unsigned)(n0 + n1), kPredThreads, smem, st>>>(in, g, pp, anchors, qc);
+    h->launches += 1;
+    CK(cudaGetLastError());
+    return PRISM_OK;
+  }
   constexpr auto k0 = predict_compress_kernel<T, 0>;
   constexpr auto k1 = predict_compress_kernel<T, 1>;
   CK(smem_limit<k0>(smem));
   CK(smem_limit<k1>(smem));
-  uint64_t n0 = tiles_in_part(g, 0), n1 = tiles_in_part(g, 1);
   CK(fork_join(
       h, st, n0 > 0, n1 > 0, [&](cudaStream_t s) { k0<<<(unsigned)n0, kPredThreads, smem, s>>>(in, g, pp, anchors, qc); },
       [&](cudaStream_t s) { k1<<<(unsigned)n1, kPredThreads, smem, s>>>(in, g, pp, anchors, qc); }));
@@ -375,11 +383,9 @@ static const PredParams<T>* params_ptr(prism_handle* h) {
 
 // ---- stage launchers ----
 
-// per_sm: extrema CTAs per SM (four fill an SM; two, with 16-byte loads, still
-// keep the copy bandwidth and leave room for the auto-tune beside them)
 template <class T>
-static int launch_extrema(prism_handle* h, const T* in, uint64_t n, cudaStream_t st, int per_sm = 4) {
-  int blocks = (int)std::min<uint64_t>((n + kExtThreads - 1) / kExtThreads, (uint64_t)h->sm_count * per_sm);
+static int launch_extrema(prism_handle* h, const T* in, uint64_t n, cudaStream_t st) {
+  int blocks = (int)std::min<uint64_t>((n + kExtThreads - 1) / kExtThreads, (uint64_t)h->sm_count * 4);
   CKA(h->ext.ensure(sizeof(T) * 2 * blocks));
   prof_begin(h, kStExtrema, st);
   extrema_kernel<T><<<blocks, kExtThreads, 0, st>>>(in, n, h->ext.as<T>());
@@ -394,59 +400,53 @@ __global__ void set_double_kernel(double* p, double v) { *p = v; }
 
 static double alpha_of(double r);
 
-// the auto-tune's error sums over the sample windows (no dependence on the
-// error bound, so it can run beside the extrema scan)
+// ints the predictor never writes but the shuffle reads
+static ZeroList code_padding(int32_t* qc, const Geometry& g) {
+  const uint64_t c3 = g.grid[2] - g.grid[3], c2 = g.grid[1] - g.grid[2], c1 = g.grid[0] - g.grid[1];
+  const uint64_t from[4] = {g.anchors + c3, g.lm_prefix[2] + c2, g.lm_prefix[1] + c1,
+                            g.lm_prefix[0] + (g.n - g.grid[0])};
+  const uint64_t to[4] = {g.lm_prefix[2], g.lm_prefix[1], g.lm_prefix[0], qc_len(g)};
+  ZeroList z;
+  for (int k = 0; k < 4; ++k) {
+    z.p[k] = qc + from[k];
+    z.n[k] = to[k] > from[k] ? to[k] - from[k] : 0;
+  }
+  return z;
+}
+
+// Auto-tune sums, extrema (mode 1) and code padding, then the decisions, the
+// range and the per-level parameters (autotune.cuh).
 template <class T>
-static int launch_autotune(prism_handle* h, const T* in, const Geometry& g, cudaStream_t st) {
-  std::vector<SampleWindow> wins = sample_grid(g.nx, g.ny, g.nz);
+static int launch_front(prism_handle* h, const T* in, const Geometry& g, int mode, double bound, cudaStream_t st) {
+  const std::vector<SampleWindow> wins = sample_grid(g.nx, g.ny, g.nz);
   const int nwin = (int)wins.size();
   CKA(h->part.ensure(sizeof(T) * 15 * std::max(nwin, 1) + 64));
-  if (nwin > 0) {
-    if (h->wins_dims[0] != g.nx || h->wins_dims[1] != g.ny || h->wins_dims[2] != g.nz) {
-      CKA(h->wins.ensure(sizeof(SampleWindow) * nwin));
-      CK(cudaMemcpyAsync(h->wins.p, wins.data(), sizeof(SampleWindow) * nwin, cudaMemcpyHostToDevice, st));
-      h->wins_dims[0] = g.nx;
-      h->wins_dims[1] = g.ny;
-      h->wins_dims[2] = g.nz;
-    }
-    prof_begin(h, kStAutotune, st);
-    autotune_kernel<T><<<dim3(nwin, 6), kAttThreads, 0, st>>>(in, g, h->wins.as<SampleWindow>(), h->part.as<T>());
-    prof_end(h, kStAutotune, st);
-    h->launches += 1;
+  if (nwin > 0 && (h->wins_dims[0] != g.nx || h->wins_dims[1] != g.ny || h->wins_dims[2] != g.nz)) {
+    CKA(h->wins.ensure(sizeof(SampleWindow) * nwin));
+    CK(cudaMemcpyAsync(h->wins.p, wins.data(), sizeof(SampleWindow) * nwin, cudaMemcpyHostToDevice, st));
+    h->wins_dims[0] = g.nx;
+    h->wins_dims[1] = g.ny;
+    h->wins_dims[2] = g.nz;
   }
-  CK(cudaGetLastError());
-  return PRISM_OK;
-}
-
-// the decisions and per-level parameters from the sums (or forced flags) and
-// the range
-template <class T>
-static int launch_params(prism_handle* h, const Geometry& g, int mode, double bound, double rel_for_alpha,
-                         const uint8_t* force_flags_dev, cudaStream_t st) {
-  const double alpha = alpha_of(rel_for_alpha);  // InterpolationPredictor.cu:2248-2271
+  const int next = mode == 1 ? (int)std::min<uint64_t>((g.n + kAttThreads - 1) / kAttThreads, (uint64_t)h->sm_count * 4)
+                             : 0;
+  CKA(h->ext.ensure(sizeof(T) * 2 * std::max(next, 1)));
   Small* s = small(h);
-  if (!force_flags_dev) {
-    const int nwin = (int)sample_grid(g.nx, g.ny, g.nz).size();
-    params_kernel<T><<<1, 32, 0, st>>>(mode, bound, &s->range, alpha, h->part.as<T>(), nwin, nullptr, 4,
-                                       reinterpret_cast<PredParams<T>*>(s->params),
-                                       reinterpret_cast<T*>(s->errors), &s->eb);
-  } else {
-    params_kernel<T><<<1, 32, 0, st>>>(mode, bound, &s->range, alpha, nullptr, 0, force_flags_dev, 4,
-                                       reinterpret_cast<PredParams<T>*>(s->params), nullptr, &s->eb);
-  }
-  h->launches += 1;
+  prof_begin(h, kStExtrema, st);
+  front_kernel<T><<<nwin * 6 + next + 4, kAttThreads, 0, st>>>(in, g, h->wins.as<SampleWindow>(), nwin * 6,
+                                                               h->part.as<T>(), next, h->ext.as<T>(),
+                                                               code_padding(h->qc.as<int32_t>(), g));
+  prof_end(h, kStExtrema, st);
+  prof_begin(h, kStAutotune, st);
+  front_params_kernel<T><<<1, kAttThreads, 0, st>>>(mode, bound, h->ext.as<T>(), next,
+                                                    alpha_of(mode == 1 ? bound : 0.0),  // :2248-2271
+                                                    h->part.as<T>(), nwin, &s->range,
+                                                    reinterpret_cast<PredParams<T>*>(s->params),
+                                                    reinterpret_cast<T*>(s->errors), &s->eb);
+  prof_end(h, kStAutotune, st);
+  h->launches += 2;
   CK(cudaGetLastError());
   return PRISM_OK;
-}
-
-template <class T>
-static int launch_autotune_params(prism_handle* h, const T* in, const Geometry& g, int mode, double bound,
-                                  double rel_for_alpha, const uint8_t* force_flags_dev, cudaStream_t st) {
-  if (!force_flags_dev) {
-    const int rc = launch_autotune<T>(h, in, g, st);
-    if (rc) return rc;
-  }
-  return launch_params<T>(h, g, mode, bound, rel_for_alpha, force_flags_dev, st);
 }
 
 static double alpha_of(double r) {
@@ -458,20 +458,6 @@ static double alpha_of(double r) {
   if (r >= e4) return a4 + (a3 - a4) * (r - e4) / (e3 - e4);
   if (r >= e5) return a5 + (a4 - a5) * (r - e5) / (e4 - e5);
   return a5;
-}
-
-// zero the code slots the predictor never writes but the shuffle reads
-static int zero_code_padding(prism_handle* h, const Geometry& g, cudaStream_t st) {
-  int32_t* qc = h->qc.as<int32_t>();
-  uint64_t c3 = g.grid[2] - g.grid[3], c2 = g.grid[1] - g.grid[2], c1 = g.grid[0] - g.grid[1];
-  uint64_t c0 = g.n - g.grid[0];
-  uint64_t segs[4][2] = {{g.anchors + c3, g.lm_prefix[2]},
-                         {g.lm_prefix[2] + c2, g.lm_prefix[1]},
-                         {g.lm_prefix[1] + c1, g.lm_prefix[0]},
-                         {g.lm_prefix[0] + c0, qc_len(g)}};
-  for (auto& s : segs)
-    if (s[1] > s[0]) CK(cudaMemsetAsync(qc + s[0], 0, (s[1] - s[0]) * sizeof(int32_t), st));
-  return PRISM_OK;
 }
 
 // rows (may be null): nonzero planes per shuffle item, for launch_encode
@@ -528,9 +514,38 @@ static int launch_inverse(prism_handle* h, const uint8_t* planes, const Geometry
 
 // Encode a plane buffer to a stream; payloads are staged in `slots` (plane
 // buffer sized; may be `planes`, which is then overwritten).  rows: from
-// launch_bitshuffle of these planes, or null.
+// launch_bitshuffle of these planes, or null.  The call's results are
+// published to the host block; trailer() runs on `trailer_ctas` CTAs beside the
+// gather, once the stream's size is known.
+struct PublishResult {
+  const Small* s;
+  HostResult* out;
+  __device__ __forceinline__ void operator()() const {
+    for (int t = threadIdx.x; t < (int)sizeof(s->params); t += blockDim.x) out->params[t] = s->params[t];
+    if (threadIdx.x == 0) {
+      out->padded_size = s->padded_size;
+      out->error_flag = s->error_flag;
+    }
+  }
+};
+struct NoTrailer {
+  __device__ __forceinline__ void operator()() const {}
+};
+template <class T>
+struct Trailer {
+  uint8_t* stream;
+  const Small* s;
+  const T* anchors;
+  uint64_t nanchors;
+  int ctas;
+  __device__ __forceinline__ void operator()() const {
+    write_trailer(stream + s->padded_size, reinterpret_cast<const PredParams<T>*>(s->params), &s->range, s->csbp, anchors,
+                  nanchors, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, (uint64_t)ctas * blockDim.x, ~0ull);
+  }
+};
+template <class F = NoTrailer>
 static int launch_encode(prism_handle* h, const uint8_t* planes, uint8_t* slots, const uint32_t* rows,
-                         const Geometry& g, uint8_t* stream, cudaStream_t st) {
+                         const Geometry& g, uint8_t* stream, cudaStream_t st, int trailer_ctas = 0, F trailer = F()) {
   Small* s = small(h);
   const EncodeJob job{planes, slots, reinterpret_cast<uint16_t*>(stream + 8)};
   int64_t* offs = h->offs.as<int64_t>();
@@ -541,9 +556,10 @@ static int launch_encode(prism_handle* h, const uint8_t* planes, uint8_t* slots,
   encode_chunks_kernel<<<blocks, kEncThreads, smem, st>>>(job, g, make_shuf_plan(g, (g.sh_grid - 1) * (int64_t)kChunk),
                                                            rows);
   scan_stream_kernel<<<(unsigned)((g.chunks + kScanItems - 1) / kScanItems), kScanThreads, 0, st>>>(
-      stream, g, offs, StreamTotals{s->csbp, &s->lossless_size, &s->padded_size, &s->error_flag});
-  gather_stream_kernel<<<(unsigned)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * 8), kEncThreads, 0, st>>>(
-      job, g, stream, offs);
+      stream, g, offs, StreamTotals{s->csbp, &s->lossless_size, &s->padded_size, &s->error_flag},
+      PublishResult{s, h->host_dev});
+  const int gather = (int)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * 8);
+  gather_stream_kernel<<<gather + trailer_ctas, kEncThreads, 0, st>>>(job, g, stream, offs, trailer_ctas, trailer);
   prof_end(h, kStEncode, st);
   h->launches += 3;
   CK(cudaGetLastError());
@@ -624,13 +640,6 @@ static int launch_decode(prism_handle* h, const uint8_t* stream, uint64_t stream
   return PRISM_OK;
 }
 
-template <class T>
-__global__ void trailer_kernel(uint8_t* stream, const uint64_t* padded, const PredParams<T>* p, const double* range,
-                               const uint64_t* csbp, const T* anchors, uint64_t nanchors) {
-  write_trailer(stream + *padded, p, range, csbp, anchors, nanchors,
-                (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x, ~0ull);
-}
-
 // the results of a pipeline call, stored into the handle's mapped host block
 __global__ void publish_result_kernel(const Small* __restrict__ s, HostResult* out) {
   const int t = threadIdx.x;
@@ -642,15 +651,20 @@ __global__ void publish_result_kernel(const Small* __restrict__ s, HostResult* o
   if (t < 16) out->errors[t] = s->errors[t];
 }
 
-static int finish(prism_handle* h, cudaStream_t st) {
-  publish_result_kernel<<<1, 256, 0, st>>>(small(h), h->host_dev);
-  h->launches += 1;
-  CK(cudaGetLastError());
+// wait for a call whose kernels published its results
+static int finish_published(prism_handle* h, cudaStream_t st) {
   CK(cudaStreamSynchronize(st));
   prof_collect(h);
   if (h->host->error_flag == 1) return fail(h, PRISM_ERR_TIMEOUT, "look-back wait exceeded its limit");
   if (h->host->error_flag == 2) return fail(h, PRISM_ERR_CORRUPT, "corrupt lossless chunk");
   return PRISM_OK;
+}
+
+static int finish(prism_handle* h, cudaStream_t st) {
+  publish_result_kernel<<<1, 256, 0, st>>>(small(h), h->host_dev);
+  h->launches += 1;
+  CK(cudaGetLastError());
+  return finish_published(h, st);
 }
 
 template <class T>
@@ -661,22 +675,7 @@ static int compress_t(prism_handle* h, const T* in, const Geometry& g, int mode,
   uint64_t need = 8 + 2 * (uint64_t)g.chunks + g.aligned_size + 8 + g.header_size;
   if (cap < need) return fail(h, PRISM_ERR_ARG, "output capacity below prism_max_container_size");
   Small* s = small(h);
-  if (mode == 1) {
-    // the extrema scan (two CTAs per SM) and the auto-tune side by side
-    int rc_ext = PRISM_OK, rc_att = PRISM_OK;
-    CK(fork_join(
-        h, st, true, true, [&](cudaStream_t x) { rc_ext = launch_extrema<T>(h, in, g.n, x, 2); },
-        [&](cudaStream_t x) { rc_att = launch_autotune<T>(h, in, g, x); }));
-    if (rc_ext) return rc_ext;
-    if (rc_att) return rc_att;
-  } else {
-    set_double_kernel<<<1, 1, 0, st>>>(&s->range, 1.0);
-    rc = launch_autotune<T>(h, in, g, st);
-    if (rc) return rc;
-  }
-  rc = launch_params<T>(h, g, mode, bound, mode == 1 ? bound : 0.0, nullptr, st);
-  if (rc) return rc;
-  rc = zero_code_padding(h, g, st);
+  rc = launch_front<T>(h, in, g, mode, bound, st);
   if (rc) return rc;
   prof_begin(h, kStPredict, st);
   rc = launch_predict<T>(h, in, g, params_ptr<T>(h), h->anchors.as<T>(), h->qc.as<int32_t>(), st);
@@ -685,15 +684,11 @@ static int compress_t(prism_handle* h, const T* in, const Geometry& g, int mode,
   rc = launch_bitshuffle(h, h->qc.as<int32_t>(), g, nb, h->planes.as<uint8_t>(),
                         h->marks.as<uint32_t>(), st);
   if (rc) return rc;
-  rc = launch_encode(h, h->planes.as<uint8_t>(), h->planes.as<uint8_t>(), h->marks.as<uint32_t>(), g, out, st);
+  const int trailer_ctas = (int)std::min<uint64_t>(64, (1040 + g.anchors * sizeof(T)) / (4 * kEncThreads) + 1);
+  rc = launch_encode(h, h->planes.as<uint8_t>(), h->planes.as<uint8_t>(), h->marks.as<uint32_t>(), g, out, st,
+                     trailer_ctas, Trailer<T>{out, s, h->anchors.as<T>(), g.anchors, trailer_ctas});
   if (rc) return rc;
-  prof_begin(h, kStTrailer, st);
-  trailer_kernel<T><<<64, 256, 0, st>>>(out, &s->padded_size, params_ptr<T>(h), &s->range, s->csbp,
-                                        h->anchors.as<T>(), g.anchors);
-  prof_end(h, kStTrailer, st);
-  h->launches += 1;
-  CK(cudaGetLastError());
-  rc = finish(h, st);
+  rc = finish_published(h, st);
   if (rc) return rc;
   *out_size = h->host->padded_size + g.header_size;
   if (flags_out) {
@@ -714,8 +709,8 @@ static int decompress_t(prism_handle* h, const uint8_t* cont, uint64_t size, con
     return fail(h, PRISM_ERR_ARG, "container trailer not aligned to the value type");
   Small* s = small(h);
   CK(cudaMemcpyAsync(&s->range, tr + 8, sizeof(double), cudaMemcpyDeviceToDevice, st));
-  params_kernel<T><<<1, 32, 0, st>>>(mode, bound, &s->range, alpha_of(mode == 1 ? bound : 0.0), nullptr, 0, tr, 4,
-                                     reinterpret_cast<PredParams<T>*>(s->params), nullptr, &s->eb);
+  params_kernel<T><<<1, 32, 0, st>>>(mode, bound, &s->range, alpha_of(mode == 1 ? bound : 0.0), tr, 4,
+                                     reinterpret_cast<PredParams<T>*>(s->params), &s->eb);
   rc = launch_decode(h, cont, size - g.header_size, g, nullptr, nullptr, h->planes.as<uint8_t>(), true, st);
   if (rc) return rc;
   rc = launch_inverse(h, h->planes.as<uint8_t>(), g, 0 /*SM*/, nullptr, nullptr, chunk_live(cont, nullptr, nullptr),
@@ -1226,9 +1221,8 @@ int prism_autotune(prism_handle* h, const void* d_in, int dtype_size, uint32_t n
   int rc = ensure_common(h, g);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  set_double_kernel<<<1, 1, 0, st>>>(&small(h)->range, 1.0);
-  rc = dtype_size == 4 ? launch_autotune_params<float>(h, (const float*)d_in, g, 0, 1.0, 0.0, nullptr, st)
-                       : launch_autotune_params<double>(h, (const double*)d_in, g, 0, 1.0, 0.0, nullptr, st);
+  rc = dtype_size == 4 ? launch_front<float>(h, (const float*)d_in, g, 0, 1.0, st)
+                       : launch_front<double>(h, (const double*)d_in, g, 0, 1.0, st);
   if (rc) return rc;
   rc = finish(h, st);
   if (rc) return rc;
@@ -1255,8 +1249,8 @@ static int predict_stage_t(prism_handle* h, const T* in, const Geometry& g, doub
   Small* s = small(h);
   CK(cudaMemcpyAsync(s->params + 200, flags, 8, cudaMemcpyHostToDevice, st));
   set_double_kernel<<<1, 1, 0, st>>>(&s->range, 1.0);
-  params_kernel<T><<<1, 32, 0, st>>>(0, eb, &s->range, alpha_of(rel_eb), nullptr, 0, s->params + 200, 4,
-                                     reinterpret_cast<PredParams<T>*>(s->params), nullptr, &s->eb);
+  params_kernel<T><<<1, 32, 0, st>>>(0, eb, &s->range, alpha_of(rel_eb), s->params + 200, 4,
+                                     reinterpret_cast<PredParams<T>*>(s->params), &s->eb);
   rc = launch_predict<T>(h, in, g, params_ptr<T>(h), anchors, codes, st);
   if (rc) return rc;
   return finish(h, st);
@@ -1282,8 +1276,8 @@ static int reconstruct_stage_t(prism_handle* h, const int32_t* codes, const T* a
   Small* s = small(h);
   CK(cudaMemcpyAsync(s->params + 200, flags, 8, cudaMemcpyHostToDevice, st));
   set_double_kernel<<<1, 1, 0, st>>>(&s->range, 1.0);
-  params_kernel<T><<<1, 32, 0, st>>>(0, eb, &s->range, alpha_of(rel_eb), nullptr, 0, s->params + 200, maxlevel,
-                                     reinterpret_cast<PredParams<T>*>(s->params), nullptr, &s->eb);
+  params_kernel<T><<<1, 32, 0, st>>>(0, eb, &s->range, alpha_of(rel_eb), s->params + 200, maxlevel,
+                                     reinterpret_cast<PredParams<T>*>(s->params), &s->eb);
   rc = old ? launch_reconstruct<T, true>(h, codes, anchors, g, params_ptr<T>(h), old, out, st)
            : launch_reconstruct<T, false>(h, codes, anchors, g, params_ptr<T>(h), nullptr, out, st);
   if (rc) return rc;
@@ -1361,7 +1355,7 @@ int prism_lossless_encode(prism_handle* h, const uint8_t* d_planes, uint32_t nx,
   rc = launch_encode(h, d_planes, h->planes.as<uint8_t>(), nullptr, g, d_stream, st);
   if (rc) return rc;
   if (comp_size_bp) CK(cudaMemcpyAsync(comp_size_bp, small(h)->csbp, 1024, cudaMemcpyDeviceToHost, st));
-  rc = finish(h, st);
+  rc = finish_published(h, st);
   if (rc) return rc;
   *size_out = h->host->padded_size;
   return PRISM_OK;

@@ -846,9 +846,16 @@ __device__ __forceinline__ void scan_stream(uint8_t* stream, const Geometry& g, 
     }
   });
 }
+// publish(): the call's results for the host, by the last CTA once its totals
+// are written
+template <class F>
 __global__ void __launch_bounds__(kScanThreads)
-scan_stream_kernel(uint8_t* stream, Geometry g, int64_t* offs, StreamTotals t) {
+scan_stream_kernel(uint8_t* stream, Geometry g, int64_t* offs, StreamTotals t, F publish) {
   scan_stream(stream, g, offs, t, blockIdx.x);
+  if (blockIdx.x == gridDim.x - 1) {
+    __syncthreads();
+    publish();
+  }
 }
 
 // Copy n bytes from an 8-byte aligned address to an arbitrarily aligned one:
@@ -890,13 +897,14 @@ struct GatherItem {
   int n;
 };
 template <class F>
-__device__ __forceinline__ void gather_items(GatherItem (&list)[kEncThreads], const uint64_t items, F find) {
+__device__ __forceinline__ void gather_items(GatherItem (&list)[kEncThreads], const uint64_t items, const int cta,
+                                             const int ncta, F find) {
   __shared__ int listed;
   const int tid = threadIdx.x;
-  for (uint64_t i0 = blockIdx.x; i0 < items; i0 += (uint64_t)gridDim.x * kEncThreads) {
+  for (uint64_t i0 = cta; i0 < items; i0 += (uint64_t)ncta * kEncThreads) {
     if (tid == 0) listed = 0;
     __syncthreads();
-    const uint64_t i = i0 + (uint64_t)tid * gridDim.x;
+    const uint64_t i = i0 + (uint64_t)tid * ncta;
     if (i < items) {
       GatherItem it;
       if (find(i, it)) list[atomicAdd(&listed, 1)] = it;
@@ -921,10 +929,17 @@ __device__ __forceinline__ bool gather_chunk(const EncodeJob& job, const Geometr
   it.src = (it.n == loc.osize ? job.planes : job.slots) + loc.base;
   return true;
 }
+// The first `front` CTAs do front(cta) instead (the trailer).
+template <class F>
 __global__ void __launch_bounds__(kEncThreads)
-gather_stream_kernel(const EncodeJob job, Geometry g, uint8_t* stream, const int64_t* __restrict__ offs) {
+gather_stream_kernel(const EncodeJob job, Geometry g, uint8_t* stream, const int64_t* __restrict__ offs, int front_ctas,
+                     F front) {
   __shared__ GatherItem list[kEncThreads];
-  gather_items(list, (uint64_t)g.chunks, [&](uint64_t i, GatherItem& it) {
+  if ((int)blockIdx.x < front_ctas) {
+    front();
+    return;
+  }
+  gather_items(list, (uint64_t)g.chunks, blockIdx.x - front_ctas, gridDim.x - front_ctas, [&](uint64_t i, GatherItem& it) {
     return gather_chunk(job, g, stream, offs, (int64_t)i, it);
   });
 }
