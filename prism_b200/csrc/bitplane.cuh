@@ -322,14 +322,11 @@ encode_chunks_kernel(const EncodeJob job, Geometry g, ShufPlan plan, const uint3
 // written by the decoder nor read here (128^3 floats at REL 1e-4: 9.4 -> 8.0
 // us; 1000x777x513 at ABS 1e-3, a third of the chunks all-zero: 620 -> 590 us,
 // 81% of the copy bandwidth for the bytes still moved).
-__global__ void __launch_bounds__(kShufWarps * 32, 4)
-inverse_bitshuffle_kernel(const uint8_t* __restrict__ planes, int32_t* __restrict__ codes, Geometry g,
-                          ShufPlan plan, int nb, const int* __restrict__ begin, const int* __restrict__ end,
-                          ChunkLive live) {
-  __shared__ __align__(16) uint32_t tile[kShufWarps][32][33];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int64_t item = (int64_t)blockIdx.x * kShufWarps + warp;
-  if (item >= plan.items) return;
+__device__ __forceinline__ void inverse_item(uint32_t (&tw)[32][33], const uint8_t* __restrict__ planes,
+                                             int32_t* __restrict__ codes, const Geometry& g, const ShufPlan& plan, int nb,
+                                             const int* __restrict__ begin, const int* __restrict__ end,
+                                             const ChunkLive& live, int64_t item) {
+  const int lane = threadIdx.x & 31;
   int level;
   int64_t local;
   locate_item(plan, item, &level, &local);
@@ -364,7 +361,6 @@ inverse_bitshuffle_kernel(const uint8_t* __restrict__ planes, int32_t* __restric
     return;
   }
   const uint8_t* base = planes + at;
-  uint32_t (&tw)[32][33] = tile[warp];
   // a[k] = transformed code 32 lane + plane_bit_code(k) (code bit b from
   // plane 31 - b, bit k of the lane's word)
   uint32_t a[32];
@@ -548,56 +544,73 @@ shuffle_last_block_kernel(const int32_t* __restrict__ codes, uint8_t* __restrict
   shuffle_last_block(codes, planes, g, nb, limit, blockIdx.x, gridDim.x);
 }
 
-// inverse of the last block (bitplane.cu:400-450 and :532-600): thread t
-// decodes positions t, t+512, ... below its own res; lanes that left the loop
-// supply 0 to the network.  begin/end (device, may be null) mask planes.
-__global__ void __launch_bounds__(512)
-inverse_last_block_kernel(const uint8_t* __restrict__ planes, int32_t* __restrict__ codes, Geometry g, int nb,
-                          const int* __restrict__ begin, const int* __restrict__ end, uint64_t limit,
-                          ChunkLive live) {
-  __shared__ uint32_t a[512];
-  __shared__ unsigned char act[512];
-  const int t = threadIdx.x;
-  const int64_t start = (g.sh_grid - 1) * (int64_t)kChunk;
-  const int64_t res = last_res_of(g, t);
-  const int64_t maxr = last_res_of(g, 0);
-  for (int64_t base = (int64_t)blockIdx.x * 512; base < maxr; base += (int64_t)gridDim.x * 512) {
-    int64_t c = start + base + t;
-    bool ac = base + t < res;
-    uint32_t v = 0;
-    if (ac) {
-      int level = 0;
-      while (level < 3 && c < g.dprefix[level]) ++level;
-      int64_t st;
-      int64_t s = place_dev(g, c, &st);
-      int lane = (int)(((c - g.dprefix[level]) & 7) << 2);
-      int lo = 0, hi = 32;
-      if (begin) { lo = begin[3 - level]; hi = end[3 - level]; }
-      if (lo < hi) {
-        const int sh[4] = {24, 8, 16, 0};
-        for (int j = 0; j < 4; ++j) {
-          uint64_t o = (uint64_t)(s + j * st);
-          if (lane + j >= lo && lane + j < hi && o < limit &&
-              !(live.sizes && live.dead(chunk_near(g, level, lane + j, (int64_t)o))))
-            v |= (uint32_t)planes[o] << sh[j];
-        }
+// inverse of the last block (bitplane.cu:400-450 and :532-600): thread t of a
+// round decodes positions t, t+512, ... below its own res; lanes that left the
+// loop supply 0 to the network.  begin/end (device, may be null) mask planes.
+// CTA `cta` of 256 threads takes half a round (the network joins eight lanes)
+// and clears the codes the block does not reach; together the CTAs cover the
+// code buffer from the block's start to its end.
+constexpr int kInvThreads = kShufWarps * 32;
+__device__ __forceinline__ void inverse_last_block(const uint8_t* __restrict__ planes, int32_t* __restrict__ codes,
+                                                   const Geometry& g, int nb, const int* __restrict__ begin,
+                                                   const int* __restrict__ end, const ChunkLive& live, int64_t count,
+                                                   int cta, uint32_t* a) {
+  static_assert(512 % kInvThreads == 0, "whole parts of a round");
+  const int64_t pos = (int64_t)cta * kInvThreads + threadIdx.x;  // from the block's start
+  const int t = (int)(pos % 512);
+  const int64_t c = (g.sh_grid - 1) * (int64_t)kChunk + pos;
+  const bool ac = pos < last_res_of(g, t);
+  uint32_t v = 0;
+  if (ac) {
+    int level = 0;
+    while (level < 3 && c < g.dprefix[level]) ++level;
+    int64_t st;
+    const int64_t s = place_dev(g, c, &st);
+    const int plane = (int)(((c - g.dprefix[level]) & 7) << 2);
+    int lo = 0, hi = 32;
+    if (begin) { lo = begin[3 - level]; hi = end[3 - level]; }
+    if (lo < hi) {
+      const int sh[4] = {24, 8, 16, 0};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint64_t o = (uint64_t)(s + j * st);
+        if (plane + j >= lo && plane + j < hi && o < g.aligned_size &&
+            !(live.sizes && live.dead(chunk_near(g, level, plane + j, (int64_t)o))))
+          v |= (uint32_t)planes[o] << sh[j];
       }
-      v = bits_inv(v);
     }
-    act[t] = ac;
-    a[t] = v;
+    v = bits_inv(v);
+  }
+  // a lane that is not active holds 0, as its partners read it
+  uint32_t* own = a + threadIdx.x;
+#pragma unroll
+  for (int step = 0; step < 3; ++step) {
+    *own = v;
     __syncthreads();
-    for (int step = 0; step < 3; ++step) {
-      int partner = t ^ (4 >> step);
-      uint32_t q = act[partner] ? a[partner] : 0u;
-      uint32_t nv = ac ? net_step(a[t], q, t & 7, step) : 0u;
-      __syncthreads();
-      a[t] = nv;
-      __syncthreads();
-    }
-    if (ac) codes[c] = sign_inverse(a[t], nb);
+    const uint32_t q = a[threadIdx.x ^ (4 >> step)];
+    v = ac ? net_step(v, q, t & 7, step) : 0u;
     __syncthreads();
   }
+  if (pos < count) codes[c] = ac ? sign_inverse(v, nb) : 0;
+}
+
+// The bulk items (kShufWarps a CTA), then the last block's CTAs over `tail`
+// codes, then (when the grid has one CTA more) publish().
+template <class F>
+__global__ void __launch_bounds__(kInvThreads, 4)
+inverse_bitshuffle_kernel(const uint8_t* __restrict__ planes, int32_t* __restrict__ codes, Geometry g,
+                          ShufPlan plan, int nb, const int* __restrict__ begin, const int* __restrict__ end,
+                          ChunkLive live, int64_t tail, F publish) {
+  __shared__ __align__(16) uint32_t tile[kShufWarps][32][33];
+  const int64_t bulk = (plan.items + kShufWarps - 1) / kShufWarps;
+  if (blockIdx.x < bulk) {
+    const int64_t item = (int64_t)blockIdx.x * kShufWarps + (threadIdx.x >> 5);
+    if (item < plan.items) inverse_item(tile[threadIdx.x >> 5], planes, codes, g, plan, nb, begin, end, live, item);
+    return;
+  }
+  const int64_t cta = blockIdx.x - bulk;
+  if (cta * kInvThreads < tail) inverse_last_block(planes, codes, g, nb, begin, end, live, tail, (int)cta, &tile[0][0][0]);
+  else publish();
 }
 
 // The plane buffer starts out holding the predictor's linear int32 codes (the

@@ -1403,15 +1403,10 @@ __device__ __forceinline__ void fetch_level0_vec(ReconSmem<T>& sm, const int32_t
   }
 }
 
-template <class T, bool PROG, int PART>
-__global__ void __launch_bounds__(kPredThreads, reconstruct_min_ctas<T, PART>())
-reconstruct_kernel(const int32_t* __restrict__ qc, const T* __restrict__ anchors, Geometry g,
-                   const PredParams<T>* __restrict__ pp, const T* old, T* out) {
-  constexpr bool EDGE = PART == 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ReconSmem<T>& sm = *reinterpret_cast<ReconSmem<T>*>(smem_raw);
-  uint32_t bi[3];
-  tile_of_block<PART>(g, bi);
+template <class T, bool PROG, bool EDGE>
+__device__ __forceinline__ void reconstruct_tile(ReconSmem<T>& sm, const int32_t* __restrict__ qc,
+                                                 const T* __restrict__ anchors, const Geometry& g, const uint32_t bi[3],
+                                                 const PredParams<T>* __restrict__ pp, const T* old, T* out) {
   TileFrame f;
   tile_frame(g, bi, f);
   const Limits<EDGE> L{f.lim};
@@ -1567,6 +1562,35 @@ reconstruct_kernel(const int32_t* __restrict__ qc, const T* __restrict__ anchors
       T v = sm.win[Win<T>::at(x, y, z)];
       out[base + x + (uint64_t)y * sy + (uint64_t)z * sz] = PROG ? Fp<T>::add(v, o[k]) : v;
     }
+  }
+}
+
+template <class T, bool PROG, int PART>
+__global__ void __launch_bounds__(kPredThreads, reconstruct_min_ctas<T, PART>())
+reconstruct_kernel(const int32_t* __restrict__ qc, const T* __restrict__ anchors, Geometry g,
+                   const PredParams<T>* __restrict__ pp, const T* old, T* out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint32_t bi[3];
+  tile_of_block<PART>(g, bi);
+  reconstruct_tile<T, PROG, PART == 1>(*reinterpret_cast<ReconSmem<T>*>(smem_raw), qc, anchors, g, bi, pp, old, out);
+}
+
+// Both parts in one launch (predict_compress_both_kernel).
+constexpr int kReconBothCtas = 5;
+template <class T, bool PROG>
+__global__ void __launch_bounds__(kPredThreads, kReconBothCtas)
+reconstruct_both_kernel(const int32_t* __restrict__ qc, const T* __restrict__ anchors, Geometry g,
+                        const PredParams<T>* __restrict__ pp, const T* old, T* out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ReconSmem<T>& sm = *reinterpret_cast<ReconSmem<T>*>(smem_raw);
+  const uint32_t edge = (uint32_t)tiles_in_part(g, 1);
+  uint32_t bi[3];
+  if (blockIdx.x < edge) {
+    tile_of_index<1>(g, blockIdx.x, bi);
+    reconstruct_tile<T, PROG, true>(sm, qc, anchors, g, bi, pp, old, out);
+  } else {
+    tile_of_index<0>(g, blockIdx.x - edge, bi);
+    reconstruct_tile<T, PROG, false>(sm, qc, anchors, g, bi, pp, old, out);
   }
 }
 

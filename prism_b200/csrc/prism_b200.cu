@@ -13,6 +13,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -346,11 +347,19 @@ static int launch_reconstruct(prism_handle* h, const int32_t* qc, const T* ancho
     return PRISM_OK;
   }
   const int smem0 = recon_smem_bytes<T>(), smem1 = recon_smem_bytes<T>();
+  const uint64_t n0 = tiles_in_part(g, 0), n1 = tiles_in_part(g, 1);
+  if (n0 > 0 && n0 + n1 <= (uint64_t)h->sm_count * kReconBothCtas) {  // one wave of the joined kernel
+    constexpr auto k = reconstruct_both_kernel<T, PROG>;
+    CK(smem_limit<k>(smem0));
+    k<<<(unsigned)(n0 + n1), kPredThreads, smem0, st>>>(qc, anchors, g, pp, old, out);
+    h->launches += 1;
+    CK(cudaGetLastError());
+    return PRISM_OK;
+  }
   constexpr auto k0 = reconstruct_kernel<T, PROG, 0>;
   constexpr auto k1 = reconstruct_kernel<T, PROG, 1>;
   CK(smem_limit<k0>(smem0));
   CK(smem_limit<k1>(smem1));
-  uint64_t n0 = tiles_in_part(g, 0), n1 = tiles_in_part(g, 1);
   CK(fork_join(
       h, st, n0 > 0, n1 > 0,
       [&](cudaStream_t s) { k0<<<(unsigned)n0, kPredThreads, smem0, s>>>(qc, anchors, g, pp, old, out); },
@@ -486,26 +495,26 @@ static int launch_bitshuffle(prism_handle* h, const int32_t* qc, const Geometry&
   return PRISM_OK;
 }
 
+struct Nothing {
+  __device__ __forceinline__ void operator()() const {}
+};
+
 // live: the dead chunks of `planes` (written by launch_decode with the same
-// one), which are not read
+// one), which are not read.  publish() runs on a CTA of its own once the
+// planes are decoded.
+template <class F = Nothing>
 static int launch_inverse(prism_handle* h, const uint8_t* planes, const Geometry& g, int nb, const int* dbegin,
-                          const int* dend, const ChunkLive& live, int32_t* qc, cudaStream_t st) {
-  int64_t start_last = (g.sh_grid - 1) * (int64_t)kChunk;
-  // positions from the last block on are only partly written: start from 0
-  uint64_t from = g.anchors + (uint64_t)start_last;
-  uint64_t to = qc_len(g);
-  if (to > from) CK(cudaMemsetAsync(qc + from, 0, (to - from) * sizeof(int32_t), st));
-  ShufPlan plan = make_shuf_plan(g, start_last);
-  int32_t* codes = qc + g.anchors;
+                          const int* dend, const ChunkLive& live, int32_t* qc, cudaStream_t st, F publish = F()) {
+  const int64_t start_last = (g.sh_grid - 1) * (int64_t)kChunk;
+  // positions from the last block on are only partly written: the others are
+  // cleared, to the end of the buffer
+  const int64_t tail = (int64_t)(qc_len(g) - g.anchors) - start_last;
+  const ShufPlan plan = make_shuf_plan(g, start_last);
+  const int64_t blocks = (plan.items + kShufWarps - 1) / kShufWarps + (tail + kInvThreads - 1) / kInvThreads +
+                         (std::is_same<F, Nothing>::value ? 0 : 1);
   prof_begin(h, kStInverse, st);
-  if (plan.items > 0) {
-    int64_t blocks = (plan.items + kShufWarps - 1) / kShufWarps;
-    inverse_bitshuffle_kernel<<<(unsigned)blocks, kShufWarps * 32, 0, st>>>(planes, codes, g, plan, nb, dbegin, dend,
-                                                                             live);
-    h->launches += 1;
-  }
-  inverse_last_block_kernel<<<last_block_rounds(g), 512, 0, st>>>(planes, codes, g, nb, dbegin, dend, g.aligned_size,
-                                                                    live);
+  inverse_bitshuffle_kernel<<<(unsigned)blocks, kInvThreads, 0, st>>>(planes, qc + g.anchors, g, plan, nb, dbegin, dend,
+                                                                      live, tail, publish);
   prof_end(h, kStInverse, st);
   h->launches += 1;
   CK(cudaGetLastError());
@@ -528,9 +537,6 @@ struct PublishResult {
     }
   }
 };
-struct NoTrailer {
-  __device__ __forceinline__ void operator()() const {}
-};
 template <class T>
 struct Trailer {
   uint8_t* stream;
@@ -543,7 +549,7 @@ struct Trailer {
                   nanchors, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, (uint64_t)ctas * blockDim.x, ~0ull);
   }
 };
-template <class F = NoTrailer>
+template <class F = Nothing>
 static int launch_encode(prism_handle* h, const uint8_t* planes, uint8_t* slots, const uint32_t* rows,
                          const Geometry& g, uint8_t* stream, cudaStream_t st, int trailer_ctas = 0, F trailer = F()) {
   Small* s = small(h);
@@ -592,14 +598,43 @@ static int launch_encode_lookback(prism_handle* h, const uint8_t* planes, const 
   return PRISM_OK;
 }
 
-// payload offsets and coded chunks of a stream (ChunkTable in `table`)
-static void launch_chunk_table(prism_handle* h, const uint8_t* stream, const Geometry& g, void* table,
-                               cudaStream_t st) {
+// payload offsets and coded chunks of a stream (ChunkTable in `table`); open()
+// runs beside it
+template <class F>
+static int launch_chunk_table(prism_handle* h, const uint8_t* stream, const Geometry& g, void* table, F open,
+                              cudaStream_t st) {
   const int64_t blocks = (g.chunks + kScanItems - 1) / kScanItems;
-  scan_chunks_kernel<<<(unsigned)blocks, kScanThreads, 0, st>>>(reinterpret_cast<const uint16_t*>(stream + 8), g,
-                                                                chunk_table(table, g.chunks));
+  scan_chunks_kernel<<<(unsigned)blocks + 1, kScanThreads, 0, st>>>(reinterpret_cast<const uint16_t*>(stream + 8), g,
+                                                                    chunk_table(table, g.chunks), open);
   h->launches += 1;
+  CK(cudaGetLastError());
+  return PRISM_OK;
 }
+
+// what a decode needs beside the chunk table: its error flag cleared, and
+// (trailer not null) the parameters from a container's trailer, whose doubles
+// may be aligned to 4 bytes only
+template <class T>
+struct OpenDecode {
+  int* err;
+  const uint8_t* trailer;
+  int mode;
+  double bound, alpha;
+  PredParams<T>* params;
+  double* range;
+  double* eb;
+  __device__ __forceinline__ void operator()() const {
+    if (threadIdx.x != 0) return;
+    *err = 0;
+    if (!trailer) return;
+    double r;
+    uint8_t* q = reinterpret_cast<uint8_t*>(&r);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) q[k] = trailer[8 + k];
+    *range = r;
+    compute_params<T>(mode, bound, &r, alpha, nullptr, 0, trailer, 4, params, nullptr, eb);
+  }
+};
 
 // The chunks of a stream an inverse shuffle need not read after launch_decode
 // of the planes [dbegin, dend) (null: all).
@@ -608,22 +643,12 @@ static ChunkLive chunk_live(const uint8_t* stream, const int* dbegin, const int*
 }
 
 // edges: the planes are only read through chunk_live, so dead chunks are left
-// alone but for their edges.  err: where chunk errors go; null = the handle's
-// flag, reset here.  table: the stream's chunk table if already built (else
-// built here).
+// alone but for their edges.  err: where chunk errors go (cleared by the
+// caller's open()).  table: the stream's chunk table.
 static int launch_decode(prism_handle* h, const uint8_t* stream, uint64_t stream_bytes, const Geometry& g,
-                         const int* dbegin, const int* dend, uint8_t* planes, bool edges, cudaStream_t st,
-                         int* err = nullptr, void* table = nullptr) {
-  Small* s = small(h);
+                         const int* dbegin, const int* dend, uint8_t* planes, bool edges, cudaStream_t st, int* err,
+                         void* table) {
   prof_begin(h, kStDecode, st);
-  if (!table) {
-    table = h->offs.p;
-    launch_chunk_table(h, stream, g, table, st);
-  }
-  if (!err) {
-    err = &s->error_flag;
-    CK(cudaMemsetAsync(err, 0, sizeof(int), st));
-  }
   size_t smem = sizeof(DecodeShared);
   int blocks = (int)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * kDecCtas);
   const ChunkTable t = chunk_table(table, g.chunks);
@@ -708,22 +733,22 @@ static int decompress_t(prism_handle* h, const uint8_t* cont, uint64_t size, con
   if (reinterpret_cast<uintptr_t>(tr) % sizeof(T))  // the anchors are read in place
     return fail(h, PRISM_ERR_ARG, "container trailer not aligned to the value type");
   Small* s = small(h);
-  CK(cudaMemcpyAsync(&s->range, tr + 8, sizeof(double), cudaMemcpyDeviceToDevice, st));
-  params_kernel<T><<<1, 32, 0, st>>>(mode, bound, &s->range, alpha_of(mode == 1 ? bound : 0.0), tr, 4,
-                                     reinterpret_cast<PredParams<T>*>(s->params), &s->eb);
-  rc = launch_decode(h, cont, size - g.header_size, g, nullptr, nullptr, h->planes.as<uint8_t>(), true, st);
+  rc = launch_chunk_table(h, cont, g, h->offs.p,
+                          OpenDecode<T>{&s->error_flag, tr, mode, bound, alpha_of(mode == 1 ? bound : 0.0),
+                                        reinterpret_cast<PredParams<T>*>(s->params), &s->range, &s->eb}, st);
+  if (rc) return rc;
+  rc = launch_decode(h, cont, size - g.header_size, g, nullptr, nullptr, h->planes.as<uint8_t>(), true, st,
+                     &s->error_flag, h->offs.p);
   if (rc) return rc;
   rc = launch_inverse(h, h->planes.as<uint8_t>(), g, 0 /*SM*/, nullptr, nullptr, chunk_live(cont, nullptr, nullptr),
-                      h->qc.as<int32_t>(), st);
+                      h->qc.as<int32_t>(), st, PublishResult{s, h->host_dev});
   if (rc) return rc;
   prof_begin(h, kStReconstruct, st);
   rc = launch_reconstruct<T, false>(h, h->qc.as<int32_t>(), reinterpret_cast<const T*>(tr + 1040), g,
                                     params_ptr<T>(h), nullptr, out, st);
   if (rc) return rc;
   prof_end(h, kStReconstruct, st);
-  h->launches += 1;
-  CK(cudaGetLastError());
-  return finish(h, st);
+  return finish_published(h, st);
 }
 
 // ---- exported API (C linkage comes from the declarations in prism_b200.h) ----
@@ -961,10 +986,18 @@ __global__ void prog_plan_kernel(const StrategyBest* __restrict__ blk, int mode,
     }
 }
 
-__global__ void prog_init_kernel(StrategyState* st, int* err) {
-  if (threadIdx.x < 4) { st->begin[threadIdx.x] = 0; st->end[threadIdx.x] = 0; }
-  if (threadIdx.x == 0) { st->maxlevel = 4; *err = 0; }
-}
+// the state before an object's first step: no planes loaded, all levels, no
+// errors (first = false: left as it is)
+struct OpenProgressive {
+  bool first;
+  StrategyState* st;
+  int* err;
+  __device__ __forceinline__ void operator()() const {
+    if (!first) return;
+    if (threadIdx.x < 4) { st->begin[threadIdx.x] = 0; st->end[threadIdx.x] = 0; }
+    if (threadIdx.x == 0) { st->maxlevel = 4; *err = 0; }
+  }
+};
 
 // the state of an object whose planes [0, end) are already reconstructed
 __global__ void prog_resume_kernel(StrategyState* st, int* err, int e0, int e1, int e2, int e3) {
@@ -980,18 +1013,23 @@ __global__ void prog_resume_kernel(StrategyState* st, int* err, int e0, int e1, 
 // end), so the total is planes [0, end) of each level, a difference of the
 // trailer's cumulative sizes (calculate_accumulate_size, analyze.hpp:118-159,
 // summed over the steps).
-__global__ void prog_publish_kernel(const StrategyState* __restrict__ st, const int* __restrict__ err,
-                                    const uint64_t* __restrict__ cum, ProgMirror* out) {
-  if (threadIdx.x != 0) return;
-  uint64_t total = 0;
-  for (int i = 0; i < 4; ++i) {
-    const int e = min(st->end[i], 32);
-    if (e > 0) total += cum[i * 32 + e - 1] - (i > 0 ? cum[i * 32 - 1] : 0);
+struct PublishProgressive {
+  const StrategyState* st;
+  const int* err;
+  const uint64_t* cum;
+  ProgMirror* out;
+  __device__ __forceinline__ void operator()() const {
+    if (threadIdx.x != 0) return;
+    uint64_t total = 0;
+    for (int i = 0; i < 4; ++i) {
+      const int e = min(st->end[i], 32);
+      if (e > 0) total += cum[i * 32 + e - 1] - (i > 0 ? cum[i * 32 - 1] : 0);
+    }
+    out->state = *st;
+    out->err = *err;
+    out->loaded = total;
   }
-  out->state = *st;
-  out->err = *err;
-  out->loaded = total;
-}
+};
 
 template <class T>
 static int progressive_step_t(prism_prog* p, double target, const T* prev, T* values, cudaStream_t st) {
@@ -1041,10 +1079,20 @@ static int progressive_step_t(prism_prog* p, double target, const T* prev, T* va
   PredParams<T>* params = reinterpret_cast<PredParams<T>*>(slot ? s->params_odd : s->params);
   if (slot) CKA(h->qc_odd.ensure(qc_len(g) * sizeof(int32_t)));
   int32_t* codes = slot ? h->qc_odd.as<int32_t>() : h->qc.as<int32_t>();
-  // ---- on the decode stream: strategy, plan, chunk offsets, decode, state
-  if (first) {  // no planes loaded, all levels, no errors
-    prog_init_kernel<<<1, 32, 0, dst>>>(ds, p->d_err);
-    h->launches += 1;
+  // ---- on the decode stream: chunk table, strategy, plan, decode, state
+  // the chunk table: once per object when it holds a slot
+  void* table = h->offs.p;
+  bool build = true;
+  if (p->slot >= 0) {
+    DevBuf& ob = h->prog_offs[p->slot];
+    build = !p->offs_ready;
+    if (build) CKA(ob.ensure(chunk_table_bytes(g.chunks)));
+    table = ob.p;
+  }
+  if (build) {
+    rc = launch_chunk_table(h, p->cont, g, table, OpenProgressive{first, ds, p->d_err}, dst);
+    if (rc) return rc;
+    p->offs_ready = p->slot >= 0;
   }
   // strategy (findStrategy_h) from the container's cumulative plane sizes;
   // it advances the object's device state in place
@@ -1057,17 +1105,6 @@ static int progressive_step_t(prism_prog* p, double target, const T* prev, T* va
                                          p->exact ? s->dec_begin : nullptr);
   prof_end(h, kStStrategy, dst);
   h->launches += 2;
-  // chunk table: once per object when it holds a slot
-  void* table = nullptr;
-  if (p->slot >= 0) {
-    DevBuf& ob = h->prog_offs[p->slot];
-    if (!p->offs_ready) {
-      CKA(ob.ensure(chunk_table_bytes(g.chunks)));
-      launch_chunk_table(h, p->cont, g, ob.p, dst);
-      p->offs_ready = true;
-    }
-    table = ob.p;
-  }
   // chunks of planes the step does not load read as zeros; the inverse
   // shuffle keeps planes [begin, end) of what was decoded
   const int* dec_begin = p->exact ? s->dec_begin : ds->begin;
@@ -1075,10 +1112,10 @@ static int progressive_step_t(prism_prog* p, double target, const T* prev, T* va
                      p->d_err, table);
   if (rc) return rc;
   // the state after the step (plane ranges, errors, bytes loaded) for the host
-  prog_publish_kernel<<<1, 32, 0, dst>>>(ds, p->d_err, csbp, p->mirror_dev);
-  h->launches += 1;
+  // beside the inverse shuffle
   rc = launch_inverse(h, h->planes.as<uint8_t>(), g, 1 /*NB*/, ds->begin, ds->end,
-                      chunk_live(p->cont, dec_begin, ds->end), codes, dst);
+                      chunk_live(p->cont, dec_begin, ds->end), codes, dst,
+                      PublishProgressive{ds, p->d_err, csbp, p->mirror_dev});
   if (rc) return rc;
   CK(cudaEventRecord(h->dec_done, dst));
   // ---- on the caller's stream: reconstruction
@@ -1442,7 +1479,11 @@ int prism_lossless_decode(prism_handle* h, const uint8_t* d_stream, uint32_t nx,
   int *db, *de;
   rc = host_range(h, begin, end, st, &db, &de);
   if (rc) return rc;
-  rc = launch_decode(h, d_stream, ~0ull, g, db, de, d_planes, false, st);
+  int* err = &small(h)->error_flag;
+  rc = launch_chunk_table(h, d_stream, g, h->offs.p, OpenDecode<float>{err, nullptr, 0, 0, 0, nullptr, nullptr, nullptr},
+                          st);
+  if (rc) return rc;
+  rc = launch_decode(h, d_stream, ~0ull, g, db, de, d_planes, false, st, err, h->offs.p);
   if (rc) return rc;
   return finish(h, st);
 }

@@ -543,8 +543,15 @@ __device__ __forceinline__ void scan_chunks(const uint16_t* __restrict__ sizes, 
   }
 }
 
+// One CTA more than the scan's does open() instead: what else a decode has to
+// have before it starts (parameters, cleared flags).
+template <class F>
 __global__ void __launch_bounds__(kScanThreads)
-scan_chunks_kernel(const uint16_t* __restrict__ sizes, Geometry g, ChunkTable t) {
+scan_chunks_kernel(const uint16_t* __restrict__ sizes, Geometry g, ChunkTable t, F open) {
+  if (blockIdx.x == gridDim.x - 1) {
+    open();
+    return;
+  }
   scan_chunks(sizes, g.chunks, blockIdx.x, [&](int64_t i, uint32_t size, uint64_t off, uint32_t rank, bool coded) {
     t.offs[i] = (int64_t)off;
     t.rank[i] = rank;
