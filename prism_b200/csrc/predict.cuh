@@ -434,9 +434,20 @@ __device__ __forceinline__ T cube_at(const T* w, int ox, int oy, int oz, bool na
 }
 
 // One level (unit U) of a tile sweep.
+// In a compression, levels 3 and 2 (U = 8, 4; at most 50 points a stage) are
+// swept by warp 0 alone, with warp barriers between their six stages: the
+// other warps wait once instead of stepping through every stage's loop and
+// barrier.  (The reconstruction, with more tiles an SM and less to do per
+// point, was 1.5% slower that way: 1885 -> 1914 us on 1000x777x513 floats.)
 template <class T, bool COMPRESS, int U, bool EDGE>
 struct LevelSweep {
   static constexpr int N = 16 / (2 * U);
+  static constexpr bool kWarp = COMPRESS && U >= 4;
+  static constexpr int kThreads = kWarp ? 32 : kPredThreads;
+  static __device__ __forceinline__ void sync() {
+    if constexpr (kWarp) __syncwarp();
+    else __syncthreads();
+  }
   T* win;
   int32_t* cw;
   Limits<EDGE> L;
@@ -488,7 +499,7 @@ struct LevelSweep {
     constexpr int total = N0 * N1 * N2;
     constexpr int A0 = AXES & 3, A1 = (AXES >> 2) & 3, A2 = (AXES >> 4) & 3;
 #pragma unroll 2
-    for (int i = threadIdx.x; i < total; i += kPredThreads) {
+    for (int i = threadIdx.x; i < total; i += kThreads) {
       const int k0 = i % N0, k1 = (i / N0) % N1, k2 = i / (N0 * N1);
       int c[3];
       c[A0] = U * (k0 * ST0 + OF0);
@@ -498,7 +509,7 @@ struct LevelSweep {
       const int wi = Win<T>::at(c[0], c[1], c[2]);
       emit(wi, c, line_at<T, U, AX, MD>(win + wi, order_of<U, EDGE, AX>(L, c[AX]), nat));
     }
-    if (SYNC) __syncthreads();
+    if (SYNC) sync();
   }
   // md faces: the point is even along axis E (dimension 0, fastest) and odd
   // along the two interpolation axes P1 (the reference's a1) and P2 (a2)
@@ -506,7 +517,7 @@ struct LevelSweep {
   __device__ __forceinline__ void faces() const {
     constexpr int total = (N + 1) * N * N;
 #pragma unroll 2
-    for (int i = threadIdx.x; i < total; i += kPredThreads) {
+    for (int i = threadIdx.x; i < total; i += kThreads) {
       const int k0 = i % (N + 1), k1 = (i / (N + 1)) % N, k2 = i / ((N + 1) * N);
       int c[3];
       c[E] = 2 * U * k0;
@@ -517,19 +528,19 @@ struct LevelSweep {
       emit(wi, c, face_at<T, U, P1, P2>(win + wi, order_of<U, EDGE, P1>(L, c[P1]), order_of<U, EDGE, P2>(L, c[P2]),
                                       nat));
     }
-    if (SYNC) __syncthreads();
+    if (SYNC) sync();
   }
   __device__ __forceinline__ void cube(bool exclusive) const {
     constexpr int total = N * N * N;
 #pragma unroll 2
-    for (int i = threadIdx.x; i < total; i += kPredThreads) {
+    for (int i = threadIdx.x; i < total; i += kThreads) {
       int c[3] = {2 * U * (i % N) + U, 2 * U * ((i / N) % N) + U, 2 * U * (i / (N * N)) + U};
       if (!pred_ok(c, exclusive)) continue;
       const int wi = Win<T>::at(c[0], c[1], c[2]);
       emit(wi, c, cube_at<T, U>(win + wi, order_of<U, EDGE, 0>(L, c[0]), order_of<U, EDGE, 1>(L, c[1]),
                              order_of<U, EDGE, 2>(L, c[2]), nat));
     }
-    __syncthreads();
+    sync();
   }
   // Level 0 of an interior tile, per-axis mode, by lines: a job predicts the
   // odd points 2j+1, j in [J0, J1), of the line along AX through window point
@@ -1067,7 +1078,7 @@ struct LevelSweep {
 template <class T, bool COMPRESS, bool EDGE, int U, int LEVEL>
 __device__ __forceinline__ void sweep_level(T* win, int32_t* cw, const AxisLimits& lim, bool zlast,
                                             const PredParams<T>& p) {
-  if (LEVEL > p.maxlevel) return;
+  if (LEVEL > p.maxlevel || (LevelSweep<T, COMPRESS, U, EDGE>::kWarp && threadIdx.x >= 32)) return;
   LevelSweep<T, COMPRESS, U, EDGE> lv{win, cw, Limits<EDGE>{lim}, zlast, p.ebr[LEVEL], p.ebx2[LEVEL]};
   lv.run(p.use_md[LEVEL] != 0, p.reverse[LEVEL] != 0);
 }
@@ -1079,6 +1090,7 @@ template <class T, bool COMPRESS, bool EDGE>
 __device__ void sweep_coarse(T* win, int32_t* cw, const AxisLimits& lim, bool zlast, const PredParams<T>& p) {
   sweep_level<T, COMPRESS, EDGE, 8, 3>(win, cw, lim, zlast, p);
   sweep_level<T, COMPRESS, EDGE, 4, 2>(win, cw, lim, zlast, p);
+  if (COMPRESS) __syncthreads();
   sweep_level<T, COMPRESS, EDGE, 2, 1>(win, cw, lim, zlast, p);
 }
 template <class T, bool COMPRESS, bool EDGE>
@@ -1179,13 +1191,28 @@ __device__ __forceinline__ int row_of(int l, int y, int z) {
   return off + (z >> l) * w + (y >> l);
 }
 
-template <class G>
+template <bool NARROW, class G>
 __device__ __forceinline__ void fill_rows(const G& g, const TileFrame& f, uint64_t* rows) {
+  // NARROW: in 32 bits where the slots allow it (rows past the field may wrap
+  // and are not used): 2% of the predictor's time, nothing in the
+  // reconstruction, which fills the table while other tiles' loads are waited
+  // for
+  const bool small = NARROW && g.n + 64 * (uint64_t)g.anchors < (1ull << 31);
   for (int r = threadIdx.x; r < kRowTable; r += kPredThreads) {
     const int l = r < 289 ? 0 : (r < 370 ? 1 : (r < 395 ? 2 : 3));
     const int w = (16 >> l) + 1, k = r - (l == 0 ? 0 : (l == 1 ? 289 : (l == 2 ? 370 : 395)));
     const int y = (k % w) << l, z = (k / w) << l;
-    rows[r] = lm_slot(g, l, (uint64_t)f.gs[0], (uint64_t)f.gs[1] + y, (uint64_t)f.gs[2] + z);
+    if (small) {  // every product and sum fits
+      const uint32_t gx = f.gs[0] >> l, gy = (f.gs[1] + y) >> l, gz = (f.gs[2] + z) >> l;
+      const uint32_t a0 = (uint32_t)g.leaps[l][0], a1 = (uint32_t)g.leaps[l][1];
+      const uint32_t b0 = (uint32_t)g.leaps[l + 1][0], b1 = (uint32_t)g.leaps[l + 1][1];
+      uint32_t s = (uint32_t)g.lm_prefix[l] + gx + gy * a0 + gz * a1 - ((gz + 1) >> 1) * b1;
+      if (!(gz & 1)) s -= ((gy + 1) >> 1) * b0;
+      if (!((gz | gy) & 1)) s -= (gx + 1) >> 1;
+      rows[r] = s;
+    } else {
+      rows[r] = lm_slot(g, l, (uint64_t)f.gs[0], (uint64_t)f.gs[1] + y, (uint64_t)f.gs[2] + z);
+    }
   }
 }
 
@@ -1289,24 +1316,28 @@ __device__ __forceinline__ void compress_tile(CompressSmem<T>& sm, const T* __re
   // emitted (on a last tile the plane at 16 lies outside the field).
   __syncthreads();
   uint64_t* rows = reinterpret_cast<uint64_t*>(sm.win);
-  fill_rows(g, f, rows);
+  fill_rows<true>(g, f, rows);
   __syncthreads();
-  // Thread t takes point (t mod 16, t / 16) of each z-plane: a row with y or z
-  // odd is all level 0 (slot rows[r] + x), the odd x of the other rows too
-  // (rows[r] + x / 2); only the even x of those go through the level lookup.
-  for (int i = tid; i < 16 * 16 * 16; i += kPredThreads) {
-    const int x = i & 15, y = (i >> 4) & 15, z = i >> 8;
-    if (!L.in_data(x, y, z)) continue;
+  // Thread t takes point (t mod 16, t / 16) of each z-plane: on an odd plane
+  // (and an odd row) the row is all level 0 (slot rows[r] + x), on the others
+  // the odd x are (rows[r] + x / 2); only the even x of those go through the
+  // level lookup.
+  static_assert(kPredThreads == 256, "a z-plane per pass");
+  const int x = tid & 15, y = tid >> 4;
+  if (!L.in_data(x, y, 0)) return;
+  const int zs = EDGE ? (f.lim.r[2] < 16 ? f.lim.r[2] : 16) : 16;
+  const bool odd_row = y & 1;
+#pragma unroll 4
+  for (int z = 0; z < zs; z += 2) {
     uint64_t slot;
-    if (((x | y | z) & 1) != 0) {
-      const int ee = ((y | z) & 1) == 0;
-      slot = rows[z * kWin + y] + (uint64_t)(x >> ee);
+    if (odd_row || (x & 1)) {
+      slot = rows[z * kWin + y] + (uint64_t)(odd_row ? x : x >> 1);
+      qc[slot] = sm.cw[cw_word(256 * z + tid)];
     } else {
       const int lv = win_level(x, y, z);
-      if (lv == 4) continue;
-      slot = slot_of(rows, lv, x, y, z);
+      if (lv < 4) qc[slot_of(rows, lv, x, y, z)] = sm.cw[cw_word(256 * z + tid)];
     }
-    qc[slot] = sm.cw[cw_word(i)];
+    if (!EDGE || z + 1 < zs) qc[rows[(z + 1) * kWin + y] + (uint64_t)x] = sm.cw[cw_word(256 * (z + 1) + tid)];
   }
 }
 
@@ -1413,7 +1444,7 @@ __device__ __forceinline__ void reconstruct_tile(ReconSmem<T>& sm, const int32_t
   const int tid = threadIdx.x;
   const int maxlevel = pp->maxlevel;
   if (tid == 0) sm.p = *pp;
-  fill_rows(g, f, sm.rows);
+  fill_rows<false>(g, f, sm.rows);
   const uint64_t sy = g.nx, sz = (uint64_t)g.nx * g.ny;
   const uint64_t base = (uint64_t)f.gs[0] + (uint64_t)f.gs[1] * sy + (uint64_t)f.gs[2] * sz;
   if (PROG) {
