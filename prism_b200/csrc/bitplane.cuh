@@ -523,18 +523,22 @@ __device__ __forceinline__ void shuffle_last_block(const int32_t* __restrict__ c
     }
     if (part) shm[t] = ac ? bits_fwd(a[t]) : 0u;
     __syncthreads();
-    int wp = ((t & 63) << 3) + (t >> 6);
-    if (part && wp < res) {
-      uint32_t w = shm[wp];
-      int64_t st;
-      int64_t s = place_dev(g, start + base + wp, &st);
-      uint8_t b[4] = {(uint8_t)(w >> 24), (uint8_t)(w >> 8), (uint8_t)(w >> 16), (uint8_t)w};
-      for (int j = 0; j < 4; ++j) {
-        uint64_t o = (uint64_t)(s + j * st);
-        if (o < limit) planes[o] = b[j];
-      }
+    // The four bytes of every word go out in step: where a word past the end
+    // of its plane spills onto bytes of the next plane that another thread of
+    // the round stores as well, the later byte of the word stands, on every
+    // run (unordered stores left it to the warps' timing).
+    const int wp = ((t & 63) << 3) + (t >> 6);
+    const bool writes = part && wp < res;
+    const uint32_t w = shm[wp];
+    int64_t st;
+    const int64_t s = place_dev(g, start + base + wp, &st);
+    const uint8_t b[4] = {(uint8_t)(w >> 24), (uint8_t)(w >> 8), (uint8_t)(w >> 16), (uint8_t)w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint64_t o = (uint64_t)(s + j * st);
+      if (writes && o < limit) planes[o] = b[j];
+      __syncthreads();
     }
-    __syncthreads();
   }
 }
 
