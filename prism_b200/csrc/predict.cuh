@@ -139,9 +139,15 @@ __device__ __forceinline__ Nb nb_even(int d, int u) {
 // pitch 16 words) falls into one or two banks; the row-dependent XOR (a
 // permutation within each row, so the block keeps its size) spreads them,
 // and a row still reads out as 16 distinct banks.
-__device__ __forceinline__ int cw_word(int i) {
-  const int y = (i >> 4) & 15, z = i >> 8;
-  return i ^ ((z + 2 * (y >> 1) + 3 * (z >> 1)) & 15);
+__device__ __forceinline__ int cw_term(int y, int z) { return z + 2 * (y >> 1) + 3 * (z >> 1); }
+__device__ __forceinline__ int cw_word(int i) { return i ^ (cw_term((i >> 4) & 15, i >> 8) & 15); }
+// The term along a job's odd points (coordinate 2j + 1 along axis J) is
+// t0 + j step(J): computed once per job instead of from each point's index
+// (1024^3 floats 5228 -> 5165 us, 384x384x256 doubles 281 -> 276 us).
+__device__ __forceinline__ int cw_term_step(int J) { return J == 0 ? 0 : (J == 1 ? 2 : 5); }
+__device__ __forceinline__ int cw_term_first(int J, int cw0) {  // of point 0 (coordinate 1)
+  const int y = (cw0 >> 4) & 15, z = cw0 >> 8;
+  return J == 2 ? cw_term(y, 0) + 1 : cw_term(y, z);
 }
 
 // FAST marks an interior tile: its whole 17^3 window lies inside the field and
@@ -572,12 +578,12 @@ struct LevelSweep {
     }
   }
   // emit_at with the point's code (compression: its original value) read
-  // beforehand
-  __device__ __forceinline__ void emit_read(int wi, int cwi, bool own, T v, T pred) const {
+  // beforehand and its code-block word known
+  __device__ __forceinline__ void emit_read(int wi, int word, bool own, T v, T pred) const {
     if (COMPRESS) {
       T rec;
       const int32_t code = quantize(v, pred, ebr, ebx2, &rec);
-      if (own) cw[cw_word(cwi)] = code;
+      if (own) cw[word] = code;
       win[wi] = rec;
     } else {
       win[wi] = Fp<T>::fma(v, ebx2, pred);
@@ -601,6 +607,7 @@ struct LevelSweep {
     constexpr int G = KIND == 1 ? 2 : 4;
     const int E2 = Win<T>::step2(J), O1 = Win<T>::one(J);  // even point e at w0 + e E2, odd point j at + O1
     const Nb nk = nb_odd<T>(K);
+    const int t0 = cw_term_first(J, cw0), dt = cw_term_step(J);
 #pragma unroll
     for (int g = 0; g < 8; g += G) {
       if (g < j0 || g >= j1) continue;
@@ -638,7 +645,7 @@ struct LevelSweep {
                                : (ok == 3 ? E::quad_l(k0[i], k1[i], k2[i]) : E::quad_r(k1[i], k2[i], k3[i]));
           pred = (oj != 4 && ok == 4) ? lk : E::half(F::add(lj, lk));
         }
-        emit_read(w0 + j * E2 + O1, cw0 + (2 * j + 1) * cs, own, v[i], pred);
+        emit_read(w0 + j * E2 + O1, (cw0 + (2 * j + 1) * cs) ^ ((t0 + j * dt) & 15), own, v[i], pred);
       }
     }
   }
@@ -649,7 +656,7 @@ struct LevelSweep {
   __device__ __forceinline__ void md_cube_job(int cy, int cz, int j0) const {
     using E = Expr<T>;
     using F = Fp<T>;
-    const int w0 = Win<T>::at(0, cy, cz), cw0 = (cz * 16 + cy) * 16;
+    const int w0 = Win<T>::at(0, cy, cz), cw0 = (cz * 16 + cy) * 16, term = cw_term(cy, cz) & 15;
     const int oy = order0(cy), oz = order0(cz);
     const Nb ny = nb_odd<T>(1), nz = nb_odd<T>(2);
     T ev[5];  // E[j0 - 1 + k] along x
@@ -694,7 +701,7 @@ struct LevelSweep {
       } else {
         pred = E::quad_r_cube(a, b, c);
       }
-      emit_read(w0 + 2 * j + 1, cw0 + 2 * j + 1, true, v[i], pred);
+      emit_read(w0 + 2 * j + 1, (cw0 + 2 * j + 1) ^ term, true, v[i], pred);
     }
   }
   // ---- level 0 of an edge tile (the last slab along some axis) by jobs ----
