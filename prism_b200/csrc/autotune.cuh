@@ -389,6 +389,7 @@ template <class T>
 __global__ void __launch_bounds__(kAttThreads)
 front_kernel(const T* __restrict__ in, Geometry g, const SampleWindow* __restrict__ wins, int natt, T* __restrict__ partial,
              int next, T* __restrict__ ext, ZeroList zero) {
+  chain_wait();
   __shared__ T win[kWinVol];
   __shared__ T red[2 * kAttThreads];
   int b = blockIdx.x;
@@ -416,6 +417,7 @@ __global__ void __launch_bounds__(kAttThreads)
 front_params_kernel(int mode, double bound, const T* __restrict__ ext, int next, double alpha,
                     const T* __restrict__ partial, int nwin, double* __restrict__ range, PredParams<T>* __restrict__ out,
                     T* __restrict__ errors_out, double* __restrict__ eb_out) {
+  chain_wait();
   __shared__ T sums[15], mns[kAttThreads / 32], mxs[kAttThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (warp == 0) {

@@ -238,6 +238,7 @@ __device__ __forceinline__ void shuffle_item(uint32_t (&tw)[32][33], const int32
 __global__ void __launch_bounds__(kShufWarps * 32)
 bitshuffle_kernel(const int32_t* __restrict__ codes, uint8_t* __restrict__ planes, Geometry g,
                   ShufPlan plan, int nb, uint32_t* rows) {
+  chain_wait();
   __shared__ uint32_t tile[kShufWarps][32][33];
   int64_t item = (int64_t)blockIdx.x * kShufWarps + (threadIdx.x >> 5);
   if (item >= plan.items) return;
@@ -301,6 +302,7 @@ __device__ __forceinline__ bool chunk_is_zero(const uint32_t* __restrict__ rows,
 // (chunk_is_zero).
 __global__ void __launch_bounds__(kEncThreads, kEncCtas)
 encode_chunks_kernel(const EncodeJob job, Geometry g, ShufPlan plan, const uint32_t* __restrict__ rows) {
+  chain_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   EncodeShared2& sh = *reinterpret_cast<EncodeShared2*>(smem_raw);
   EncodeItem(&list)[kEncThreads] = *reinterpret_cast<EncodeItem(*)[kEncThreads]>(smem_raw + sizeof(EncodeShared2));
@@ -545,6 +547,7 @@ __device__ __forceinline__ void shuffle_last_block(const int32_t* __restrict__ c
 __global__ void __launch_bounds__(512)
 shuffle_last_block_kernel(const int32_t* __restrict__ codes, uint8_t* __restrict__ planes, Geometry g,
                           int nb, uint64_t limit) {
+  chain_wait();
   shuffle_last_block(codes, planes, g, nb, limit, blockIdx.x, gridDim.x);
 }
 
@@ -666,6 +669,7 @@ __device__ __forceinline__ void leftover_fill(uint8_t* __restrict__ planes, cons
 
 __global__ void leftover_fill_kernel(uint8_t* __restrict__ planes, const int32_t* __restrict__ qc, Geometry g,
                                      const RangeList ranges, int nranges) {
+  chain_wait();
   for (int r = blockIdx.x; r < nranges; r += gridDim.x) leftover_fill(planes, qc, g, ranges.r[r].start, ranges.r[r].len);
 }
 

@@ -170,6 +170,7 @@ template <class T>
 __global__ void __launch_bounds__(kFlatWarps * 32)
 flat_compress_kernel(const T* __restrict__ data, Geometry g, const PredParams<T>* __restrict__ pp,
                      T* __restrict__ anchors, int32_t* __restrict__ qc) {
+  chain_wait();
   __shared__ T win[kFlatWarps][kFlatWin];
   const uint32_t tile = blockIdx.x * kFlatWarps + (threadIdx.x >> 5);
   if (tile < g.ax * g.ay) flat_compress_tile(win[threadIdx.x >> 5], data, g, tile, pp, anchors, qc);

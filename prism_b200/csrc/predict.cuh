@@ -14,6 +14,7 @@
 // results equal the reference build bit for bit.
 #pragma once
 #include <type_traits>
+#include "chain.cuh"
 #include "fp.cuh"
 #include "geometry.h"
 
@@ -1375,6 +1376,7 @@ template <class T>
 __global__ void __launch_bounds__(kPredThreads, 4)
 predict_compress_both_kernel(const T* __restrict__ data, Geometry g, const PredParams<T>* __restrict__ pp,
                              T* __restrict__ anchors, int32_t* __restrict__ qc) {
+  chain_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CompressSmem<T>& sm = *reinterpret_cast<CompressSmem<T>*>(smem_raw);
   const uint32_t edge = (uint32_t)tiles_in_part(g, 1);

@@ -311,7 +311,7 @@ template <class T>
 static int launch_predict(prism_handle* h, const T* in, const Geometry& g, const PredParams<T>* pp, T* anchors,
                           int32_t* qc, cudaStream_t st) {
   if (is_flat(g)) {  // a 3-D tile would spend a CTA on 256 points (flat.cuh)
-    flat_compress_kernel<T><<<(unsigned)flat_ctas(g), kFlatWarps * 32, 0, st>>>(in, g, pp, anchors, qc);
+    CK(launch_chained(flat_compress_kernel<T>, (unsigned)flat_ctas(g), kFlatWarps * 32, 0, st, in, g, pp, anchors, qc));
     h->launches += 1;
     CK(cudaGetLastError());
     return PRISM_OK;
@@ -321,7 +321,7 @@ static int launch_predict(prism_handle* h, const T* in, const Geometry& g, const
   if (n0 > 0 && n0 + n1 <= (uint64_t)h->sm_count * 4) {  // one wave of the joined kernel
     constexpr auto k = predict_compress_both_kernel<T>;
     CK(smem_limit<k>(smem));
-    k<<<(unsigned)(n0 + n1), kPredThreads, smem, st>>>(in, g, pp, anchors, qc);
+    CK(launch_chained(k, (unsigned)(n0 + n1), kPredThreads, smem, st, in, g, pp, anchors, qc));
     h->launches += 1;
     CK(cudaGetLastError());
     return PRISM_OK;
@@ -442,16 +442,14 @@ static int launch_front(prism_handle* h, const T* in, const Geometry& g, int mod
   CKA(h->ext.ensure(sizeof(T) * 2 * std::max(next, 1)));
   Small* s = small(h);
   prof_begin(h, kStExtrema, st);
-  front_kernel<T><<<nwin * 6 + next + 4, kAttThreads, 0, st>>>(in, g, h->wins.as<SampleWindow>(), nwin * 6,
-                                                               h->part.as<T>(), next, h->ext.as<T>(),
-                                                               code_padding(h->qc.as<int32_t>(), g));
+  CK(launch_chained(front_kernel<T>, nwin * 6 + next + 4, kAttThreads, 0, st, in, g, h->wins.as<SampleWindow>(), nwin * 6,
+                    h->part.as<T>(), next, h->ext.as<T>(), code_padding(h->qc.as<int32_t>(), g)));
   prof_end(h, kStExtrema, st);
   prof_begin(h, kStAutotune, st);
-  front_params_kernel<T><<<1, kAttThreads, 0, st>>>(mode, bound, h->ext.as<T>(), next,
-                                                    alpha_of(mode == 1 ? bound : 0.0),  // :2248-2271
-                                                    h->part.as<T>(), nwin, &s->range,
-                                                    reinterpret_cast<PredParams<T>*>(s->params),
-                                                    reinterpret_cast<T*>(s->errors), &s->eb);
+  CK(launch_chained(front_params_kernel<T>, 1, kAttThreads, 0, st, mode, bound, h->ext.as<T>(), next,
+                    alpha_of(mode == 1 ? bound : 0.0),  // :2248-2271
+                    h->part.as<T>(), nwin, &s->range, reinterpret_cast<PredParams<T>*>(s->params),
+                    reinterpret_cast<T*>(s->errors), &s->eb));
   prof_end(h, kStAutotune, st);
   h->launches += 2;
   CK(cudaGetLastError());
@@ -478,17 +476,19 @@ static int launch_bitshuffle(prism_handle* h, const int32_t* qc, const Geometry&
   int nr = fill_ranges(g, plan, rng.r, kMaxRanges);
   prof_begin(h, kStShuffle, st);
   if (nr > 0) {
-    leftover_fill_kernel<<<nr, 256, 0, st>>>(planes, qc, g, rng, nr);
+    CK(launch_chained(leftover_fill_kernel, nr, 256, 0, st, planes, qc, g, rng, nr));
     h->launches += 1;
   }
   const int32_t* codes = qc + g.anchors;
   bool last_last = last_block_lands_last(g);
-  if (!last_last) shuffle_last_block_kernel<<<shuffle_last_block_grid(g), 512, 0, st>>>(codes, planes, g, nb, g.aligned_size);
+  if (!last_last)
+    CK(launch_chained(shuffle_last_block_kernel, shuffle_last_block_grid(g), 512, 0, st, codes, planes, g, nb, g.aligned_size));
   if (plan.items > 0) {
     int64_t blocks = (plan.items + kShufWarps - 1) / kShufWarps;
-    bitshuffle_kernel<<<(unsigned)blocks, kShufWarps * 32, 0, st>>>(codes, planes, g, plan, nb, rows);
+    CK(launch_chained(bitshuffle_kernel, (unsigned)blocks, kShufWarps * 32, 0, st, codes, planes, g, plan, nb, rows));
   }
-  if (last_last) shuffle_last_block_kernel<<<shuffle_last_block_grid(g), 512, 0, st>>>(codes, planes, g, nb, g.aligned_size);
+  if (last_last)
+    CK(launch_chained(shuffle_last_block_kernel, shuffle_last_block_grid(g), 512, 0, st, codes, planes, g, nb, g.aligned_size));
   prof_end(h, kStShuffle, st);
   h->launches += 1 + (plan.items > 0);
   CK(cudaGetLastError());
@@ -559,13 +559,14 @@ static int launch_encode(prism_handle* h, const uint8_t* planes, uint8_t* slots,
   CK(smem_limit<encode_chunks_kernel>(smem));
   const int blocks = (int)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * kEncCtas);
   prof_begin(h, kStEncode, st);
-  encode_chunks_kernel<<<blocks, kEncThreads, smem, st>>>(job, g, make_shuf_plan(g, (g.sh_grid - 1) * (int64_t)kChunk),
-                                                           rows);
-  scan_stream_kernel<<<(unsigned)((g.chunks + kScanItems - 1) / kScanItems), kScanThreads, 0, st>>>(
-      stream, g, offs, StreamTotals{s->csbp, &s->lossless_size, &s->padded_size, &s->error_flag},
-      PublishResult{s, h->host_dev});
+  CK(launch_chained(encode_chunks_kernel, blocks, kEncThreads, smem, st, job, g,
+                    make_shuf_plan(g, (g.sh_grid - 1) * (int64_t)kChunk), rows));
+  CK(launch_chained(scan_stream_kernel<PublishResult>, (unsigned)((g.chunks + kScanItems - 1) / kScanItems), kScanThreads, 0,
+                    st, stream, g, offs, StreamTotals{s->csbp, &s->lossless_size, &s->padded_size, &s->error_flag},
+                    PublishResult{s, h->host_dev}));
   const int gather = (int)std::min<int64_t>(g.chunks, (int64_t)h->sm_count * 8);
-  gather_stream_kernel<<<gather + trailer_ctas, kEncThreads, 0, st>>>(job, g, stream, offs, trailer_ctas, trailer);
+  CK(launch_chained(gather_stream_kernel<F>, gather + trailer_ctas, kEncThreads, 0, st, job, g, stream, offs, trailer_ctas,
+                    trailer));
   prof_end(h, kStEncode, st);
   h->launches += 3;
   CK(cudaGetLastError());

@@ -20,6 +20,7 @@
 // size table; one CTA per coded chunk rebuilds the bitmaps from the tail and
 // expands the bytes (a fill-forward is an inclusive popcount prefix).
 #pragma once
+#include "chain.cuh"
 #include "geometry.h"
 
 namespace prism_b200 {
@@ -858,6 +859,7 @@ __device__ __forceinline__ void scan_stream(uint8_t* stream, const Geometry& g, 
 template <class F>
 __global__ void __launch_bounds__(kScanThreads)
 scan_stream_kernel(uint8_t* stream, Geometry g, int64_t* offs, StreamTotals t, F publish) {
+  chain_wait();
   scan_stream(stream, g, offs, t, blockIdx.x);
   if (blockIdx.x == gridDim.x - 1) {
     __syncthreads();
@@ -957,6 +959,7 @@ template <class F>
 __global__ void __launch_bounds__(kEncThreads)
 gather_stream_kernel(const EncodeJob job, Geometry g, uint8_t* stream, const int64_t* __restrict__ offs, int front_ctas,
                      F front) {
+  chain_wait();
   __shared__ GatherItem list[kEncThreads];
   if ((int)blockIdx.x < front_ctas) {
     front();
