@@ -198,10 +198,10 @@ int prism_inverse_bitshuffle(prism_handle* h, const uint8_t* d_planes, uint32_t 
 int prism_lossless_encode(prism_handle* h, const uint8_t* d_planes, uint32_t nx, uint32_t ny,
                           uint32_t nz, uint8_t* d_stream, uint64_t capacity, uint64_t* size_out,
                           uint64_t comp_size_bp[128], void* stream);
-/* Self-test of the failure detection in the encoder's look-back (no
+/* Self-test of the failure detection in the one-launch encoder's look-back (no
  * counterpart in the reference, whose decoupled look-back in zbpc_encode,
  * src/encoder/zbpc.cu:113-153, spins without a limit).  Runs the kernels of
- * prism_lossless_encode with the chunk tickets starting at 1, so chunk 0 never
+ * prism_lossless_encode_static with the chunk tickets starting at 1, so chunk 0 never
  * publishes its size and every wait that reaches it gives up after
  * `spin_limit` polls (about 64 ns apart).  Returns PRISM_ERR_TIMEOUT when the
  * bounded wait works; the stream bytes it leaves are meaningless.  The handle

@@ -579,6 +579,16 @@ scan_chunks_kernel(const uint16_t* __restrict__ sizes, Geometry g, ChunkTable t,
 // and chunks that the bit-plane shuffle knows to be zero are never read.  The
 // one-launch encoder stays for the entry point that has no scratch to put
 // payloads in.
+//
+// us for the one-launch encoder -> encode + scan + gather: 384x384x256 double
+// at REL 1e-6 (151 MB of planes, 86 MB out) 172 -> 40 + 5 + 32 (floor 36);
+// 1024^3 float sparse at ABS 1e-3 (two thirds of 262 K chunks coded) 3468 ->
+// 1360 + 22 + 123; 32 uneven float fields 482 -> 85 + 6 + 40.  The encode
+// launch waits on the latency of a chunk's loads and barriers; five CTAs an
+// SM (48 registers) against 4 / 6 / 8: 40 / 40 / 43 / 67 us and
+// 1360 / 1369 / 1422 / 2139 us on the first two.  Fetching the next chunk with
+// asynchronous copies meanwhile was slower (1675-1851 us: the staging adds to
+// the shared-memory traffic).
 constexpr int kEncThreads = 256, kEncWarps = kEncThreads / 32, kEncCtas = 5;
 
 struct EncodeJob {
@@ -918,6 +928,7 @@ __device__ __forceinline__ void gather_items(GatherItem (&list)[kEncThreads], co
                                              const int ncta, F find) {
   __shared__ int listed[2];  // short payloads from the front of the list, the others from its end
   const int tid = threadIdx.x;
+  const int short_max = items <= (uint64_t)ncta ? 0 : kWarpPayload;  // one payload a CTA: by the CTA
   for (uint64_t i0 = cta; i0 < items; i0 += (uint64_t)ncta * kEncThreads) {
     if (tid < 2) listed[tid] = 0;
     __syncthreads();
@@ -925,14 +936,12 @@ __device__ __forceinline__ void gather_items(GatherItem (&list)[kEncThreads], co
     if (i < items) {
       GatherItem it;
       if (find(i, it)) {
-        if (it.n <= kWarpPayload) list[atomicAdd(&listed[0], 1)] = it;
+        if (it.n <= short_max) list[atomicAdd(&listed[0], 1)] = it;
         else list[kEncThreads - 1 - atomicAdd(&listed[1], 1)] = it;
       }
     }
     __syncthreads();
-    const int few = items <= (uint64_t)ncta ? listed[0] : 0;  // at most one a CTA
-    for (int k = few + (tid >> 5); k < listed[0]; k += kEncWarps) gather_copy<32>(list[k].dst, list[k].src, list[k].n);
-    for (int k = 0; k < few; ++k) gather_copy<kEncThreads>(list[k].dst, list[k].src, list[k].n);
+    for (int k = tid >> 5; k < listed[0]; k += kEncWarps) gather_copy<32>(list[k].dst, list[k].src, list[k].n);
     for (int k = 0; k < listed[1]; ++k) {
       const GatherItem& it = list[kEncThreads - 1 - k];
       gather_copy<kEncThreads>(it.dst, it.src, it.n);
