@@ -164,42 +164,6 @@ struct EncodeShared {
   int csz;
 };
 
-// repetition elimination of `n` (<= 2048) bitmap bytes held in shared memory:
-// kept bytes go to out[pos..], flags to bmo; returns the kept count
-__device__ __forceinline__ int re_encode_block(const uint8_t* bm, int n, uint8_t* out, int pos,
-                                               uint8_t* bmo, int* scratch) {
-  // each thread takes 4 consecutive bytes (n = 2048) or 1 byte (n <= 512)
-  int per = n > kZThreads ? 4 : 1;
-  int i0 = threadIdx.x * per;
-  int flags = 0;
-  if (i0 < n) {
-    for (int k = 0; k < per; ++k) {
-      int i = i0 + k;
-      uint8_t prev = i == 0 ? 0 : bm[i - 1];
-      flags |= (bm[i] != prev) << k;
-    }
-  }
-  int total;
-  int off = block_excl_scan(__popc(flags), scratch, &total);
-  if (i0 < n) {
-    for (int k = 0; k < per; ++k)
-      if ((flags >> k) & 1) out[pos + off++] = bm[i0 + k];
-  }
-  // flags -> bitmap bytes (bit i of the whole map = flag of byte i)
-  if (per == 4) {
-    // 4 flags per thread, 2 threads per output byte
-    uint32_t f = (uint32_t)flags;
-    uint32_t other = __shfl_down_sync(0xffffffffu, f, 1);
-    if ((threadIdx.x & 1) == 0 && i0 < n) bmo[i0 / 8] = (uint8_t)(f | (other << 4));
-  } else {
-    uint32_t bal = __ballot_sync(0xffffffffu, flags & 1);
-    int lane = threadIdx.x & 31;
-    if ((lane & 7) == 0 && i0 < n) bmo[i0 / 8] = (uint8_t)(bal >> lane);
-  }
-  __syncthreads();
-  return total;
-}
-
 // Copy n bytes from shared memory to an arbitrarily aligned global address:
 // head bytes, then aligned 32-bit words (each assembled from two aligned
 // shared words), then the tail.
