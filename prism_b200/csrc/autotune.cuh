@@ -194,11 +194,10 @@ __device__ __forceinline__ void autotune_window(T* win, T* red, const T* __restr
 // alpha/beta and, when `partial` is given, the auto-tune decisions (:2306-2355)
 // from the window sums.  Flags otherwise come from `flags_in` (a container).
 template <class T>
-__device__ __forceinline__ void compute_params(int mode, double bound, const double* __restrict__ range, double alpha,
-                                               const T* __restrict__ partial, int nwin,
-                                               const uint8_t* __restrict__ flags_in, int maxlevel,
+__device__ __forceinline__ void compute_params(int mode, double bound, const double* range, double alpha,
+                                               const T* partial, int nwin, const uint8_t* flags_in, int maxlevel,
                                                PredParams<T>* __restrict__ out, T* __restrict__ errors_out,
-                                               double* __restrict__ eb_out, const T* __restrict__ sums = nullptr) {
+                                               double* __restrict__ eb_out, const T* sums = nullptr) {
   using F = Fp<T>;
   PredParams<T> p;
   double eb = mode == 1 ? __dmul_rn(bound, *range) : bound;
@@ -414,8 +413,8 @@ front_kernel(const T* __restrict__ in, Geometry g, const SampleWindow* __restric
 // decides.  next = 0: the range is 1 (an absolute bound).
 template <class T>
 __global__ void __launch_bounds__(kAttThreads)
-front_params_kernel(int mode, double bound, const T* __restrict__ ext, int next, double alpha,
-                    const T* __restrict__ partial, int nwin, double* __restrict__ range, PredParams<T>* __restrict__ out,
+front_params_kernel(int mode, double bound, const T* ext, int next, double alpha,
+                    const T* partial, int nwin, double* __restrict__ range, PredParams<T>* __restrict__ out,
                     T* __restrict__ errors_out, double* __restrict__ eb_out) {
   chain_wait();
   __shared__ T sums[15], mns[kAttThreads / 32], mxs[kAttThreads / 32];

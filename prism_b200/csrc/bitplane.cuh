@@ -175,7 +175,7 @@ __device__ __forceinline__ void locate_item(const ShufPlan& s, int64_t item, int
 // each plane's word of lane l is its 4 bytes of the plane row: one
 // contiguous 128-byte warp store per plane.
 // One warp work item of the forward shuffle (tw: the warp's staging tile).
-__device__ __forceinline__ void shuffle_item(uint32_t (&tw)[32][33], const int32_t* __restrict__ codes,
+__device__ __forceinline__ void shuffle_item(uint32_t (&tw)[32][33], const int32_t* codes,
                                              uint8_t* __restrict__ planes, const Geometry& g, const ShufPlan& plan,
                                              int nb, int64_t item, uint32_t* rows_out) {
   const int lane = threadIdx.x & 31;
@@ -194,7 +194,7 @@ __device__ __forceinline__ void shuffle_item(uint32_t (&tw)[32][33], const int32
 #pragma unroll
     for (int it = 0; it < 32; ++it) {
       const int idx = it * 32 + lane;
-      c[it] = idx < count ? __ldg(src + idx) : 0;
+      c[it] = idx < count ? src[idx] : 0;
     }
 #pragma unroll
     for (int it = 0; it < 32; ++it) {
@@ -236,7 +236,7 @@ __device__ __forceinline__ void shuffle_item(uint32_t (&tw)[32][33], const int32
 }
 
 __global__ void __launch_bounds__(kShufWarps * 32)
-bitshuffle_kernel(const int32_t* __restrict__ codes, uint8_t* __restrict__ planes, Geometry g,
+bitshuffle_kernel(const int32_t* codes, uint8_t* __restrict__ planes, Geometry g,
                   ShufPlan plan, int nb, uint32_t* rows) {
   chain_wait();
   __shared__ uint32_t tile[kShufWarps][32][33];
@@ -253,7 +253,7 @@ bitshuffle_kernel(const int32_t* __restrict__ codes, uint8_t* __restrict__ plane
 // words that block spills past a plane change nothing.  (Per-chunk flags
 // raised by the shuffle instead would be stored to by 128 items a chunk at
 // about the same time; those stores alone took nine times the shuffle.)
-__device__ __forceinline__ bool chunk_is_zero(const uint32_t* __restrict__ rows, const Geometry& g, const ShufPlan& plan,
+__device__ __forceinline__ bool chunk_is_zero(const uint32_t* rows, const Geometry& g, const ShufPlan& plan,
                                               const ChunkLoc& loc) {
   if (!rows) return false;
   int l = loc.level, p = (int)loc.plane;
@@ -287,7 +287,7 @@ __device__ __forceinline__ bool chunk_is_zero(const uint32_t* __restrict__ rows,
       static_assert(kShufCodes / 8 == 1 << 7, "bytes of a plane per item");
 #pragma unroll 4
       for (int64_t i = i0 & ~(int64_t)3; i < i1; i += 4) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(rows + i));
+        const uint4 v = *reinterpret_cast<const uint4*>(rows + i);
         uint32_t any = (i >= i0 ? v.x : 0u) | (i + 1 >= i0 && i + 1 < i1 ? v.y : 0u) |
                        (i + 2 >= i0 && i + 2 < i1 ? v.z : 0u) | (i + 3 < i1 ? v.w : 0u);
         if ((any >> (31 - p)) & 1u) return false;
@@ -301,7 +301,7 @@ __device__ __forceinline__ bool chunk_is_zero(const uint32_t* __restrict__ rows,
 // The chunks of a plane buffer (encode_items), all-zero ones by `rows`
 // (chunk_is_zero).
 __global__ void __launch_bounds__(kEncThreads, kEncCtas)
-encode_chunks_kernel(const EncodeJob job, Geometry g, ShufPlan plan, const uint32_t* __restrict__ rows) {
+encode_chunks_kernel(const EncodeJob job, Geometry g, ShufPlan plan, const uint32_t* rows) {
   chain_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   EncodeShared2& sh = *reinterpret_cast<EncodeShared2*>(smem_raw);
@@ -496,7 +496,7 @@ __device__ __forceinline__ int64_t place_dev(const Geometry& g, int64_t c, int64
   return (idx >> 3) + g.dstride[level] * ((idx & 7) << 2) + g.daprefix[level];
 }
 
-__device__ __forceinline__ void shuffle_last_block(const int32_t* __restrict__ codes, uint8_t* __restrict__ planes,
+__device__ __forceinline__ void shuffle_last_block(const int32_t* codes, uint8_t* __restrict__ planes,
                                                    const Geometry& g, int nb, uint64_t limit, int cta, int ncta) {
   __shared__ uint32_t a[512];
   __shared__ uint32_t shm[512];
@@ -545,7 +545,7 @@ __device__ __forceinline__ void shuffle_last_block(const int32_t* __restrict__ c
 }
 
 __global__ void __launch_bounds__(512)
-shuffle_last_block_kernel(const int32_t* __restrict__ codes, uint8_t* __restrict__ planes, Geometry g,
+shuffle_last_block_kernel(const int32_t* codes, uint8_t* __restrict__ planes, Geometry g,
                           int nb, uint64_t limit) {
   chain_wait();
   shuffle_last_block(codes, planes, g, nb, limit, blockIdx.x, gridDim.x);
@@ -635,7 +635,7 @@ struct RangeList {
 
 // One range by one CTA, a thread per code: the (up to) four bytes of a code
 // come from one slot lookup, in 32-bit arithmetic where the field allows it.
-__device__ __forceinline__ void leftover_fill(uint8_t* __restrict__ planes, const int32_t* __restrict__ qc,
+__device__ __forceinline__ void leftover_fill(uint8_t* __restrict__ planes, const int32_t* qc,
                                               const Geometry& g, const uint64_t start, const uint64_t len) {
   const uint64_t w0 = start >> 2, w1 = (start + len + 3) >> 2;
   const bool small = g.n >> 32 == 0;
@@ -667,7 +667,7 @@ __device__ __forceinline__ void leftover_fill(uint8_t* __restrict__ planes, cons
   }
 }
 
-__global__ void leftover_fill_kernel(uint8_t* __restrict__ planes, const int32_t* __restrict__ qc, Geometry g,
+__global__ void leftover_fill_kernel(uint8_t* __restrict__ planes, const int32_t* qc, Geometry g,
                                      const RangeList ranges, int nranges) {
   chain_wait();
   for (int r = blockIdx.x; r < nranges; r += gridDim.x) leftover_fill(planes, qc, g, ranges.r[r].start, ranges.r[r].len);

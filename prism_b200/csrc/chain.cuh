@@ -7,8 +7,17 @@ namespace prism_b200 {
 
 // First statement of every kernel launched with launch_chained: lets the next
 // kernel of the stream be set up beside this one, then waits until the
-// previous one has completed and its writes are visible.  (A no-op in a plain
-// launch.)
+// previous one has completed and its writes are visible.  (The wait is a
+// no-op in a plain launch.)
+//
+// A chained kernel's life overlaps the stores of the kernels before it, so
+// what any kernel of the call writes is not read-only for that life: such
+// data is read with ordinary loads, never through __ldg or a `const
+// __restrict__` pointer (both let the compiler use the non-coherent path and
+// move the load above the wait).  Only the caller's field may be read that
+// way: the calls that read it begin with a plain launch, so the field is
+// complete before any chained kernel starts.
+// tests/test_chained_loads.py holds the sources to this.
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

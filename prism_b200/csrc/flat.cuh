@@ -168,7 +168,7 @@ __device__ __forceinline__ void flat_compress_tile(T* win, const T* __restrict__
 
 template <class T>
 __global__ void __launch_bounds__(kFlatWarps * 32)
-flat_compress_kernel(const T* __restrict__ data, Geometry g, const PredParams<T>* __restrict__ pp,
+flat_compress_kernel(const T* __restrict__ data, Geometry g, const PredParams<T>* pp,
                      T* __restrict__ anchors, int32_t* __restrict__ qc) {
   chain_wait();
   __shared__ T win[kFlatWarps][kFlatWin];

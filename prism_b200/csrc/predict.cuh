@@ -1264,8 +1264,8 @@ struct ReconSmem {
 // reads `sm` from a previous tile.
 template <class T, bool EDGE, class G = Geometry>
 __device__ __forceinline__ void compress_tile(CompressSmem<T>& sm, const T* __restrict__ data, const G& g,
-                                              const uint32_t bi[3], const PredParams<T>* __restrict__ pp,
-                                              T* __restrict__ anchors, int32_t* __restrict__ qc) {
+                                              const uint32_t bi[3], const PredParams<T>* pp, T* __restrict__ anchors,
+                                              int32_t* __restrict__ qc) {
   TileFrame f;
   tile_frame(g, bi, f);
   const Limits<EDGE> L{f.lim};
@@ -1374,7 +1374,7 @@ predict_compress_kernel(const T* __restrict__ data, Geometry g, const PredParams
 // last end and two gaps of 8 us around them.
 template <class T>
 __global__ void __launch_bounds__(kPredThreads, 4)
-predict_compress_both_kernel(const T* __restrict__ data, Geometry g, const PredParams<T>* __restrict__ pp,
+predict_compress_both_kernel(const T* __restrict__ data, Geometry g, const PredParams<T>* pp,
                              T* __restrict__ anchors, int32_t* __restrict__ qc) {
   chain_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];

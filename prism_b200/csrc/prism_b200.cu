@@ -442,8 +442,10 @@ static int launch_front(prism_handle* h, const T* in, const Geometry& g, int mod
   CKA(h->ext.ensure(sizeof(T) * 2 * std::max(next, 1)));
   Small* s = small(h);
   prof_begin(h, kStExtrema, st);
-  CK(launch_chained(front_kernel<T>, nwin * 6 + next + 4, kAttThreads, 0, st, in, g, h->wins.as<SampleWindow>(), nwin * 6,
-                    h->part.as<T>(), next, h->ext.as<T>(), code_padding(h->qc.as<int32_t>(), g)));
+  // plain: nothing of the call starts before the caller's work on `in` has ended
+  front_kernel<T><<<nwin * 6 + next + 4, kAttThreads, 0, st>>>(in, g, h->wins.as<SampleWindow>(), nwin * 6,
+                                                               h->part.as<T>(), next, h->ext.as<T>(),
+                                                               code_padding(h->qc.as<int32_t>(), g));
   prof_end(h, kStExtrema, st);
   prof_begin(h, kStAutotune, st);
   CK(launch_chained(front_params_kernel<T>, 1, kAttThreads, 0, st, mode, bound, h->ext.as<T>(), next,

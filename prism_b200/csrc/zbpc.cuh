@@ -434,7 +434,7 @@ constexpr int kScanThreads = 1024, kScanPer = 4, kScanItems = kScanThreads * kSc
 // which costs less than a second launch or a wait on the CTAs before it.
 // each(i, size, off, rank, coded) sees every chunk of the CTA.
 template <class F>
-__device__ __forceinline__ void scan_chunks(const uint16_t* __restrict__ sizes, const int64_t n, const int cta, F each) {
+__device__ __forceinline__ void scan_chunks(const uint16_t* sizes, const int64_t n, const int cta, F each) {
   __shared__ unsigned long long warp_tot[32], prior_b[32];
   __shared__ unsigned prior_c[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -442,7 +442,7 @@ __device__ __forceinline__ void scan_chunks(const uint16_t* __restrict__ sizes, 
   const bool vec = (reinterpret_cast<uintptr_t>(sizes) & 7) == 0;  // four sizes a load
   auto four = [&](int64_t i, uint32_t (&v)[4]) {
     if (vec && i + 4 <= n) {
-      const uint2 q = __ldg(reinterpret_cast<const uint2*>(sizes + i));
+      const uint2 q = *reinterpret_cast<const uint2*>(sizes + i);
       v[0] = q.x & 0xffffu;
       v[1] = q.x >> 16;
       v[2] = q.y & 0xffffu;
@@ -846,7 +846,7 @@ scan_stream_kernel(uint8_t* stream, Geometry g, int64_t* offs, StreamTotals t, F
 // from two source words, loaded once: the second is the next lane's), four in
 // flight, then the tail.
 template <int LANES>
-__device__ __forceinline__ void gather_copy(uint8_t* dst, const uint8_t* __restrict__ src, int n) {
+__device__ __forceinline__ void gather_copy(uint8_t* dst, const uint8_t* src, int n) {
   const int tid = LANES == 32 ? threadIdx.x & 31 : threadIdx.x, lane = threadIdx.x & 31;
   int head = (int)((4 - ((uintptr_t)dst & 3)) & 3);
   if (head > n) head = n;
@@ -860,8 +860,8 @@ __device__ __forceinline__ void gather_copy(uint8_t* dst, const uint8_t* __restr
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int w = w0 + k * LANES;
-      lo[k] = w < have ? __ldg(sw + w) : 0u;
-      hi[k] = (lane == 31 && w + 1 < have) ? __ldg(sw + w + 1) : 0u;
+      lo[k] = w < have ? sw[w] : 0u;
+      hi[k] = (lane == 31 && w + 1 < have) ? sw[w + 1] : 0u;
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -930,7 +930,7 @@ __device__ __forceinline__ bool gather_chunk(const EncodeJob& job, const Geometr
 // The first `front` CTAs do front(cta) instead (the trailer).
 template <class F>
 __global__ void __launch_bounds__(kEncThreads)
-gather_stream_kernel(const EncodeJob job, Geometry g, uint8_t* stream, const int64_t* __restrict__ offs, int front_ctas,
+gather_stream_kernel(const EncodeJob job, Geometry g, uint8_t* stream, const int64_t* offs, int front_ctas,
                      F front) {
   chain_wait();
   __shared__ GatherItem list[kEncThreads];
