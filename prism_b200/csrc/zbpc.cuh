@@ -1120,8 +1120,12 @@ zbpc_decode_kernel(const uint8_t* __restrict__ stream, uint64_t stream_bytes, co
       int64_t cb = 0;
       for (int i = 3; i > l; --i) cb += g.chunks_level[i];
       const int64_t cpp = g.chunks_level[l] >> 5;
-      s = cs = cb + lo * cpp;
-      e = ce = cb + hi * cpp;
+      s = cb + lo * cpp;
+      e = cb + hi * cpp;
+      // a range may name planes past the level's 32 (or below 0): no other
+      // level's chunks are selected by them
+      cs = cb + (lo < 0 ? 0 : (lo > 32 ? 32 : lo)) * cpp;
+      ce = cb + (hi < 0 ? 0 : (hi > 32 ? 32 : hi)) * cpp;
       const int64_t a = g.daprefix[l] + (int64_t)lo * g.dstride[l], b = g.daprefix[l] + (int64_t)hi * g.dstride[l];
       const int64_t lim = (int64_t)g.aligned_size;
       if (a < b && a < lim) {
@@ -1131,8 +1135,6 @@ zbpc_decode_kernel(const uint8_t* __restrict__ stream, uint64_t stream_bytes, co
       }
       s = s < 0 ? 0 : (s > chunks ? chunks : s);
       e = e < s ? s : (e > chunks ? chunks : e);
-      cs = cs < 0 ? 0 : (cs > chunks ? chunks : cs);
-      ce = ce < cs ? cs : (ce > chunks ? chunks : ce);
     }
     range_start[l] = s;
     range_len[l] = e - s;
