@@ -639,6 +639,7 @@ __device__ __forceinline__ void leftover_fill(uint8_t* __restrict__ planes, cons
                                               const Geometry& g, const uint64_t start, const uint64_t len) {
   const uint64_t w0 = start >> 2, w1 = (start + len + 3) >> 2;
   const bool small = g.n >> 32 == 0;
+  const bool words = (reinterpret_cast<uintptr_t>(planes) & 3) == 0;  // a caller's buffer may lie anywhere
   for (uint64_t i = w0 + threadIdx.x; i < w1; i += blockDim.x) {
     uint32_t code = 0;
     if (i < g.n) {
@@ -657,7 +658,7 @@ __device__ __forceinline__ void leftover_fill(uint8_t* __restrict__ planes, cons
       if ((x & 15) | (y & 15) | (z & 15)) code = (uint32_t)qc[level_major_index(g, x, y, z)];
     }
     const uint64_t b = 4 * i;
-    if (b >= start && b + 4 <= start + len) {
+    if (words && b >= start && b + 4 <= start + len) {
       *reinterpret_cast<uint32_t*>(planes + b) = code;
     } else {
 #pragma unroll
