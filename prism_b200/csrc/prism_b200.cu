@@ -378,8 +378,6 @@ static int ensure_common(prism_handle* h, const Geometry& g) {
   ++h->epoch;
   CKA(h->qc.ensure(qc_len(g) * sizeof(int32_t)));
   CKA(h->planes.ensure(g.aligned_size + 64));
-  CKA(h->marks.ensure(marks_bytes(g)));
-  CKA(h->offs.ensure(chunk_table_bytes(g.chunks)));
   CKA(h->anchors.ensure(g.anchors * 8 + 64));
   CKA(h->small.ensure(sizeof(Small)));
   return PRISM_OK;
@@ -700,6 +698,8 @@ static int compress_t(prism_handle* h, const T* in, const Geometry& g, int mode,
                       uint8_t* out, uint64_t cap, uint64_t* out_size, uint8_t* flags_out, cudaStream_t st) {
   int rc = ensure_common(h, g);
   if (rc) return rc;
+  CKA(h->marks.ensure(marks_bytes(g)));
+  CKA(h->offs.ensure(chunk_table_bytes(g.chunks)));
   uint64_t need = 8 + 2 * (uint64_t)g.chunks + g.aligned_size + 8 + g.header_size;
   if (cap < need) return fail(h, PRISM_ERR_ARG, "output capacity below prism_max_container_size");
   Small* s = small(h);
@@ -731,6 +731,7 @@ static int decompress_t(prism_handle* h, const uint8_t* cont, uint64_t size, con
                         double bound, T* out, cudaStream_t st) {
   int rc = ensure_common(h, g);
   if (rc) return rc;
+  CKA(h->offs.ensure(chunk_table_bytes(g.chunks)));
   if (size < g.header_size + 8 + 2 * (uint64_t)g.chunks) return fail(h, PRISM_ERR_CORRUPT, "container too small");
   const uint8_t* tr = cont + (size - g.header_size);
   if (reinterpret_cast<uintptr_t>(tr) % sizeof(T))  // the anchors are read in place
@@ -1084,15 +1085,10 @@ static int progressive_step_t(prism_prog* p, double target, const T* prev, T* va
   int32_t* codes = slot ? h->qc_odd.as<int32_t>() : h->qc.as<int32_t>();
   // ---- on the decode stream: chunk table, strategy, plan, decode, state
   // the chunk table: once per object when it holds a slot
-  void* table = h->offs.p;
-  bool build = true;
-  if (p->slot >= 0) {
-    DevBuf& ob = h->prog_offs[p->slot];
-    build = !p->offs_ready;
-    if (build) CKA(ob.ensure(chunk_table_bytes(g.chunks)));
-    table = ob.p;
-  }
-  if (build) {
+  DevBuf& ob = p->slot >= 0 ? h->prog_offs[p->slot] : h->offs;
+  if (!p->offs_ready) CKA(ob.ensure(chunk_table_bytes(g.chunks)));
+  void* table = ob.p;
+  if (!p->offs_ready) {
     rc = launch_chunk_table(h, p->cont, g, table, OpenProgressive{first, ds, p->d_err}, dst);
     if (rc) return rc;
     p->offs_ready = p->slot >= 0;
@@ -1392,6 +1388,7 @@ int prism_lossless_encode(prism_handle* h, const uint8_t* d_planes, uint32_t nx,
   int rc = ensure_common(h, g);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
+  CKA(h->offs.ensure(chunk_table_bytes(g.chunks)));
   rc = launch_encode(h, d_planes, h->planes.as<uint8_t>(), nullptr, g, d_stream, st);
   if (rc) return rc;
   if (comp_size_bp) CK(cudaMemcpyAsync(comp_size_bp, small(h)->csbp, 1024, cudaMemcpyDeviceToHost, st));
@@ -1411,6 +1408,7 @@ int prism_lossless_wait_selftest(prism_handle* h, const uint8_t* d_planes, uint3
   int rc = ensure_common(h, g);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
+  CKA(h->marks.ensure(marks_bytes(g)));
   rc = launch_encode_lookback(h, d_planes, g, d_stream, st, 1, spin_limit);
   if (rc) return rc;
   return finish(h, st);
@@ -1482,6 +1480,7 @@ int prism_lossless_decode(prism_handle* h, const uint8_t* d_stream, uint32_t nx,
   int *db, *de;
   rc = host_range(h, begin, end, st, &db, &de);
   if (rc) return rc;
+  CKA(h->offs.ensure(chunk_table_bytes(g.chunks)));
   int* err = &small(h)->error_flag;
   rc = launch_chunk_table(h, d_stream, g, h->offs.p, OpenDecode<float>{err, nullptr, 0, 0, 0, nullptr, nullptr, nullptr},
                           st);

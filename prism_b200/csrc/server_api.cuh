@@ -85,12 +85,12 @@ struct SrvRequest {
 constexpr int kPlanBatch = 32;
 
 // Handle workspace one slot needs for a field (what prism_progressive_step
-// allocates: codes, planes, chunk status and two chunk tables, anchors, small
-// state).
+// allocates: codes, planes, chunk table, anchors, small state).  The table's
+// 28 bytes a chunk are counted as 24: the rest is 1/8000 of the workspace.
 uint64_t srv_workspace_bytes(uint32_t nx, uint32_t ny, uint32_t nz, int tsize) {
   Geometry g;
   make_geometry(nx, ny, nz, tsize, &g);
-  uint64_t b = qc_len(g) * 4 + g.aligned_size + 64 + marks_bytes(g) + (uint64_t)g.chunks * 2 * kChunkTableBytes + g.anchors * 16 + 65536;
+  uint64_t b = qc_len(g) * 4 + g.aligned_size + 64 + (uint64_t)g.chunks * 24 + g.anchors * 16 + 65536;
   return b + b / 8;
 }
 
@@ -413,7 +413,8 @@ int prism_server_add_field(prism_server* s, const void* container, uint64_t size
   for (size_t i = 0; i < s->handles.size(); ++i) {
     std::lock_guard<std::mutex> slk(*s->slot_mu[i]);
     prism_handle* h = s->handles[i];
-    if (ensure_common(h, g) != PRISM_OK || h->zero_anchors.ensure(g.anchors * 8 + 64) != cudaSuccess) {
+    if (ensure_common(h, g) != PRISM_OK || h->prog_offs[0].ensure(chunk_table_bytes(g.chunks)) != cudaSuccess ||
+        h->zero_anchors.ensure(g.anchors * 8 + 64) != cudaSuccess) {
       lk.lock();
       s->used -= size;
       cudaFree(f.d_cont);
