@@ -214,10 +214,14 @@ int prism_lossless_wait_selftest(prism_handle* h, const uint8_t* d_planes, uint3
  * 200-260): on some shapes the block stops short of the end of the code space
  * (trailing codes decode as 0), and on many small shapes its zero words past
  * the end of the last level-0 plane land on the first bytes of the next
- * planes (leading level-0 codes lose their low bits).  The container bytes
- * stay identical to the reference's, so the points of these codes are
- * reconstructed from a wrong code and may miss the bound.  0 for shapes
- * without the effect.  Geometry only; no device work. */
+ * planes (leading level-0 codes lose bits).  The container bytes stay
+ * identical to the reference's, so the points of these codes are
+ * reconstructed from a wrong code and may miss the bound.  Where a zero word
+ * and a real one of the same round of the block share a byte (1-D fields of
+ * 530 to 797 values, 2-D ones of about as many) the reference's bytes depend
+ * on the timing of its warps; here byte j of every word is stored before byte
+ * j + 1, always.  0 for shapes without the effect.  Geometry only; no device
+ * work. */
 uint64_t prism_lost_codes(uint32_t nx, uint32_t ny, uint32_t nz);
 /* Lossless stream -> planes.  With begin/end (host, both or neither), only
  * the chunks of planes [begin[3-l], end[3-l]) of each level are decoded; of

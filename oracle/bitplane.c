@@ -89,14 +89,14 @@ static int64_t place(const or_geom* g, int64_t c, int* level_out) {
   return (idx >> 3) + g->dstride[level] * ((idx & 7) << 2) + g->daprefix[level];
 }
 
-static void write_word(uint8_t* planes, const or_geom* g, int64_t c, uint32_t a) {
+static void write_byte(uint8_t* planes, const or_geom* g, int64_t c, uint32_t a, int j) {
+  static const int shift[4] = {24, 8, 16, 0};
   int level;
   int64_t s = place(g, c, &level);
-  int64_t st = g->dstride[level];
-  planes[s] = (uint8_t)(a >> 24);
-  planes[s + st] = (uint8_t)(a >> 8);
-  planes[s + 2 * st] = (uint8_t)(a >> 16);
-  planes[s + 3 * st] = (uint8_t)a;
+  planes[s + j * g->dstride[level]] = (uint8_t)(a >> shift[j]);
+}
+static void write_word(uint8_t* planes, const or_geom* g, int64_t c, uint32_t a) {
+  for (int j = 0; j < 4; ++j) write_byte(planes, g, c, a, j);
 }
 
 /* The 8-lane network with some lanes inactive: an inactive lane keeps 0 in
@@ -169,6 +169,13 @@ void or_bitshuffle(const int32_t* qc, const or_geom* g, int bt, uint8_t* planes)
   if (lbl) last_block_fwd(in, g, bt, planes);
 }
 
+/* Order of the stores of one round of the last block where a zero word past
+ * the end of its plane spills onto a byte that another thread of the round
+ * stores (some fields of about 513 to 1023 values): 0 = byte j of every word
+ * before byte j + 1, as warps in step store them; 1 = word after word.  The
+ * reference's own outcome is a race between its warps. */
+int or_last_block_by_words = 0;
+
 /* last block (bitplane.cu:200-260), thread by thread */
 static void last_block_fwd(const int32_t* in, const or_geom* g, int bt, uint8_t* planes) {
   int64_t start = (g->sh_grid - 1) * CS;
@@ -194,11 +201,14 @@ static void last_block_fwd(const int32_t* in, const or_geom* g, int bt, uint8_t*
       for (int l = 0; l < 8; ++l)
         if (part[l]) shm[grp * 8 + l] = o[l];
     }
-    for (int t = 0; t < TPB; ++t) {
-      if (base >= ares[t]) continue;
-      int write_pos = ((t & 63) << 3) + (t >> 6);
-      if (write_pos < res[t]) write_word(planes, g, start + base + write_pos, shm[write_pos]);
-    }
+    for (int step = 0; step < (or_last_block_by_words ? 1 : 4); ++step)
+      for (int t = 0; t < TPB; ++t) {
+        if (base >= ares[t]) continue;
+        int write_pos = ((t & 63) << 3) + (t >> 6);
+        if (write_pos >= res[t]) continue;
+        if (or_last_block_by_words) write_word(planes, g, start + base + write_pos, shm[write_pos]);
+        else write_byte(planes, g, start + base + write_pos, shm[write_pos], step);
+      }
   }
 }
 

@@ -111,6 +111,8 @@ void or_reconstruct_f64(const int32_t* qc, const double* anchors, const or_geom*
  * scratch bytes, exactly as the reference reuses that buffer). */
 void or_bitshuffle(const int32_t* qc, const or_geom* g, int bt, uint8_t* planes);
 extern int or_shuffle_last_block_last;
+/* order of the stores within a round of the last block (see bitplane.c) */
+extern int or_last_block_by_words;
 /* Inverse (:262-430) -> qc+anchors codes. */
 void or_inverse_bitshuffle(const uint8_t* planes, const or_geom* g, int bt, int32_t* qc);
 /* Progressive inverse, NB only (:433-601). */

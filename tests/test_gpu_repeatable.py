@@ -1,6 +1,7 @@
-"""Containers are the same on every call, on the sizes where threads of one
-round of the last shuffle block store to the same bytes (1-D fields of 513 to
-1023 values), alone and in a batch."""
+"""Containers are the same on every call, on 1-D fields around the sizes where
+threads of one round of the last shuffle block store to the same bytes (530 to
+797 values), alone and in a batch.  (Against the oracle, 2-D sizes among them:
+test_last_block_order.py.)"""
 import numpy as np
 import pytest
 
