@@ -1,11 +1,12 @@
-"""Failure detection on the GPU without a fault: the lossless encoder's
+"""Failure detection on the GPU without a fault: the one-launch encoder's
 look-back wait gives up after a bounded number of polls.
 
-prism_lossless_wait_selftest runs the encoder with its chunk tickets starting
+prism_lossless_wait_selftest runs that encoder with its chunk tickets starting
 at 1, so chunk 0 never publishes its size and the waits that reach it run
 out.  The call must come back with PRISM_ERR_TIMEOUT within milliseconds (the
-kernel sets an error flag and returns; nothing hangs), and the next normal
-encode on the same handle must give the same stream as before."""
+kernel sets an error flag and returns; nothing hangs).  Afterwards the handle's
+own encoder (three launches, no waits) and the one-launch encoder of
+prism_lossless_encode_static both give the stream from before."""
 import ctypes as C
 import time
 
@@ -38,6 +39,13 @@ def test_lookback_wait_runs_out_and_handle_recovers():
         assert rc == 0, P.lib().prism_last_error(h.ptr)
         return bytes(d_stream[: size.value].cpu().numpy())
 
+    def encode_static():  # the kernel whose wait ran out, on its own scratch
+        d_stream.zero_()
+        rc = l.prism_lossless_encode_static(C.c_void_p(d_planes.data_ptr()), nx, ny, nz, C.c_void_p(d_stream.data_ptr()),
+                                            cap, C.byref(size), None, st)
+        assert rc == 0
+        return bytes(d_stream[: size.value].cpu().numpy())
+
     before = encode()
     torch.cuda.synchronize()
     t0 = time.perf_counter()
@@ -49,6 +57,11 @@ def test_lookback_wait_runs_out_and_handle_recovers():
     assert b"look-back" in l.prism_last_error(h.ptr)
     after = encode()
     assert after == before
+    assert encode_static() == before
+    # and the self-test's own reset: it runs out again in the same way
+    assert l.prism_lossless_wait_selftest(h.ptr, C.c_void_p(d_planes.data_ptr()), nx, ny, nz,
+                                          C.c_void_p(d_stream.data_ptr()), cap, 2000, st) == -4
+    assert encode() == before
     # bad arguments are refused before any device work
     assert l.prism_lossless_wait_selftest(h.ptr, C.c_void_p(d_planes.data_ptr()), nx, ny, nz,
                                           C.c_void_p(d_stream.data_ptr()), cap, 0, st) == -1
