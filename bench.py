@@ -249,7 +249,9 @@ STAGE_BYTES = None
 
 def stage_algorithmic_bytes(n, tsize, aligned, cont_bytes, loaded_fraction):
     """Algorithmic HBM bytes per launch of each stage: what the stage must read
-    and write at least (inputs once, outputs once)."""
+    and write at least (inputs once, outputs once).  "extrema" also holds the
+    auto-tune windows (a few tiles read again), "autotune" only their fold;
+    the trailer is written in "encode" (1 KB and the anchors, not counted)."""
     codes = 4 * n
     return {
         "extrema": n * tsize,

@@ -69,7 +69,11 @@ const char* prism_last_error(const prism_handle* h);
  * accumulates device milliseconds per stage.  prism_stage_times copies up to n
  * accumulators (order: extrema, autotune, predict, shuffle, encode, trailer,
  * strategy, decode, inverse shuffle, reconstruct), returns the stage count and
- * clears them when reset != 0.  No counterpart in the reference, which times
+ * clears them when reset != 0.  In a compression, "extrema" is its first
+ * launch (the auto-tune windows, the extrema scan of a relative bound and the
+ * clearing of the code padding), "autotune" the one-CTA launch that folds them
+ * into the parameters, and "encode" includes the trailer, which is written
+ * beside the payloads: the "trailer" slot stays 0.  No counterpart in the reference, which times
  * its stages with blocking GPUTimer pairs (include/utils/timer.hpp:21-30).
  * prism_profile_stages times only the stages whose bit (1 << index, order
  * above) is set in mask: each timing event drains the stream, so timing

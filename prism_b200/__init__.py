@@ -136,6 +136,9 @@ def lost_codes(nx, ny, nz):
     Geometry only."""
     return int(lib().prism_lost_codes(nx, ny, nz))
 
+# In a compression "extrema" is the first launch (auto-tune windows, extrema scan,
+# code padding), "autotune" the parameters from it, and "encode" includes the
+# trailer ("trailer" stays 0).
 STAGES = ["extrema", "autotune", "predict", "shuffle", "encode", "trailer", "strategy", "decode",
           "inverse_shuffle", "reconstruct"]
 

@@ -25,8 +25,10 @@ __device__ __forceinline__ void chain_wait() {
 
 // Launch with programmatic stream serialisation: the kernel's CTAs may be
 // resident before the previous kernel of the stream has ended (it then waits
-// in chain_wait), which hides part of the 2-3 us between dependent kernels.  The
-// compression's nine launches: 64x48x40 float 99.8 -> 95.5 us, 128^3 108 -> 102
+// in chain_wait), which hides part of the 2-3 us between dependent kernels.  A
+// compression's launches after the first (nine launches in all for one-plane
+// fields and up to four tiles an SM; above, ten, the predictor's two plain ones
+// between a fork and a join): 64x48x40 float 99.8 -> 95.5 us, 128^3 108 -> 102
 // us, 384x384x256 double 602 -> 589 us.  The decompression's four gained
 // nothing (128^3 64.4 -> 68.0 us) and are plain launches.
 template <class... KArgs, class... Args>

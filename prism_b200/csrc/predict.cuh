@@ -1371,7 +1371,10 @@ predict_compress_kernel(const T* __restrict__ data, Geometry g, const PredParams
 // whose tiles are all on the GPU at once, where a second stream's events cost
 // more than the wider register budget of the joined kernel: the two parts of
 // a 64x48x40 float field (12 and 16 us) took 19 us from the first start to the
-// last end and two gaps of 8 us around them.
+// last end and two gaps of 8 us around them.  A whole compression with two
+// launches and with one, just below the limit (592 tiles, 64x64x592): float 124
+// -> 113 us, double 120 -> 114.  Above it, one launch would still take 1-8 us
+// less up to 2048 tiles and as much at 2304.
 template <class T>
 __global__ void __launch_bounds__(kPredThreads, 4)
 predict_compress_both_kernel(const T* __restrict__ data, Geometry g, const PredParams<T>* pp,
@@ -1615,7 +1618,11 @@ reconstruct_kernel(const int32_t* __restrict__ qc, const T* __restrict__ anchors
   reconstruct_tile<T, PROG, PART == 1>(*reinterpret_cast<ReconSmem<T>*>(smem_raw), qc, anchors, g, bi, pp, old, out);
 }
 
-// Both parts in one launch (predict_compress_both_kernel).
+// Both parts in one launch, as predict_compress_both_kernel.  A whole
+// decompression with two launches and with one, just below the limit (740 tiles,
+// 64x80x592): float 85 -> 76 us (61x77x590: 105 -> 80), double level (82-87
+// either way; its two progressive steps 171 -> 168).  Above it, one launch would
+// take 3-18 us less up to 1536 tiles and as much at 2304.
 constexpr int kReconBothCtas = 5;
 template <class T, bool PROG>
 __global__ void __launch_bounds__(kPredThreads, kReconBothCtas)

@@ -318,7 +318,7 @@ static int launch_predict(prism_handle* h, const T* in, const Geometry& g, const
   }
   const int smem = compress_smem_bytes<T>();
   const uint64_t n0 = tiles_in_part(g, 0), n1 = tiles_in_part(g, 1);
-  if (n0 > 0 && n0 + n1 <= (uint64_t)h->sm_count * 4) {  // one wave of the joined kernel
+  if (n0 > 0 && n0 + n1 <= (uint64_t)h->sm_count * 4) {  // one wave (predict_compress_both_kernel)
     constexpr auto k = predict_compress_both_kernel<T>;
     CK(smem_limit<k>(smem));
     CK(launch_chained(k, (unsigned)(n0 + n1), kPredThreads, smem, st, in, g, pp, anchors, qc));
@@ -348,7 +348,7 @@ static int launch_reconstruct(prism_handle* h, const int32_t* qc, const T* ancho
   }
   const int smem0 = recon_smem_bytes<T>(), smem1 = recon_smem_bytes<T>();
   const uint64_t n0 = tiles_in_part(g, 0), n1 = tiles_in_part(g, 1);
-  if (n0 > 0 && n0 + n1 <= (uint64_t)h->sm_count * kReconBothCtas) {  // one wave of the joined kernel
+  if (n0 > 0 && n0 + n1 <= (uint64_t)h->sm_count * kReconBothCtas) {  // one wave (reconstruct_both_kernel)
     constexpr auto k = reconstruct_both_kernel<T, PROG>;
     CK(smem_limit<k>(smem0));
     k<<<(unsigned)(n0 + n1), kPredThreads, smem0, st>>>(qc, anchors, g, pp, old, out);
@@ -677,7 +677,8 @@ __global__ void publish_result_kernel(const Small* __restrict__ s, HostResult* o
   if (t < 16) out->errors[t] = s->errors[t];
 }
 
-// wait for a call whose kernels published its results
+// wait for a call whose kernels published its results (flag 1 is raised by the
+// one-launch encoder's look-back only: prism_lossless_wait_selftest)
 static int finish_published(prism_handle* h, cudaStream_t st) {
   CK(cudaStreamSynchronize(st));
   prof_collect(h);
@@ -1573,8 +1574,10 @@ int prism_find_strategy_batch(prism_handle* h, int n, const uint64_t* comp_size_
 // ---------------------------------------------------------------------------
 // Lossless encode without any allocation (prism_lossless_encode_static).
 //
-// Same kernels as prism_lossless_encode, but the look-back status words, the
-// chunk ticket, the error flag and the small results live in one file-scope
+// The one-launch encoder (zbpc_encode_kernel), which needs no place for
+// payloads: same stream as prism_lossless_encode, whose three launches stage
+// them in the handle's plane buffer.  The look-back status words, the chunk
+// ticket, the error flag and the small results live in one file-scope
 // device array instead of a handle's workspace, so the call allocates nothing.
 // The array is shared by every call in the process on a given device: calls
 // whose device work overlaps (different streams, different host threads) race
