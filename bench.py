@@ -431,7 +431,7 @@ def run_prism(args, world, rank, local):
     # ---- roofline of the dominant stage ----
     peak, peak_kind = measured_peak()
     aligned = int(lib.prism_plane_buffer_size(nx, ny, nz))
-    alg = stage_algorithmic_bytes(n, 8, aligned, cont_bytes, 1.0)
+    alg = stage_algorithmic_bytes(n, 8, aligned, cont_bytes, 1.0 / len(TARGETS))  # the steps load the planes once in all
     dom = max((k for k in stage if stage[k][1] > 0), key=lambda k: stage[k][0])
     dom_ms, dom_n = stage_timed[dom] if stage_timed.get(dom, (0, 0))[1] > 0 else stage[dom]
     achieved = alg[dom] * dom_n / (dom_ms / 1e3) / 1e9 if dom_ms > 0 else 0.0
